@@ -695,6 +695,7 @@ static int prefill_gemm(cuqwen_engine* e, int mode, const __half* x, const Mat* 
     const void* w[3] = {nullptr, nullptr, nullptr}; int rows[3] = {0, 0, 0};
     for (int m = 0; m < nmat; ++m) { w[m] = mats[m]->w; rows[m] = mats[m]->rows; a.s[m] = mats[m]->s; }
     a.out_h = (__half*)out; a.out_f = (float*)out; a.T = T; a.K = mats[0]->cols; a.ldo = ldo; a.mode = mode; a.err = t_err;
+    a.pdl = !(e->p.flags & CUQWEN_FLAG_NO_PDL);
     PK(launch_prefill_gemm(e->p.quant, a, x, w, rows, nmat, e->stream));
     return CUQWEN_OK;
 }
@@ -788,15 +789,16 @@ extern "C" int cuqwen_prefill(cuqwen_engine* e, const int* tokens, int n_tokens,
     const size_t kv_layer = (size_t)e->n_kv_l * p.max_seq_len * p.head_dim;
     const float eps = __half2float(__float2half(p.norm_eps));
     const int ldqkv = qd + 2 * kd;
+    const LaunchCfg cfg{e->stream, e->sms, !(p.flags & CUQWEN_FLAG_NO_PDL)};
     CK(cudaMemsetAsync(&e->ctl->pad[0], 0, 4, e->stream));
     CK(cudaEventRecord(e->ev0, e->stream));
     for (int c0 = 0; c0 < n_tokens; c0 += C) {
         const int T = n_tokens - c0 < C ? n_tokens - c0 : C, pos = pos0 + c0;
         CK(cudaMemcpyAsync(e->pf_tok, tokens + c0, (size_t)T * 4, cudaMemcpyHostToDevice, e->stream));
-        PK(launch_pf_embed(e->embed, e->pf_tok, e->pf_x, T, p.dim, e->stream));
+        PK(launch_pf_embed(e->embed, e->pf_tok, e->pf_x, T, p.dim, LaunchCfg{e->stream, e->sms, false}));       // it follows a copy
         for (int l = 0; l < p.n_layers; ++l) {
             const Layer& L = e->layers[l];
-            PK(launch_pf_rmsnorm(e->pf_x, L.in_norm, e->pf_xn, T, p.dim, eps, e->stream));
+            PK(launch_pf_rmsnorm(e->pf_x, L.in_norm, e->pf_xn, T, p.dim, eps, cfg));
             const Mat* qkv[3] = {&L.q, &L.k, &L.v}, *om[1] = {&L.o}, *gu[2] = {&L.gate, &L.up}, *dm[1] = {&L.down};
             if (int r = prefill_gemm(e, PF_OUT_F32, e->pf_xn, qkv, 3, e->pf_qkv, T, ldqkv)) return r;        // one launch: q, k, v side by side
             PfRopeArgs ra; memset(&ra, 0, sizeof ra);
@@ -804,15 +806,15 @@ extern "C" int cuqwen_prefill(cuqwen_engine* e, const int* tokens, int n_tokens,
             ra.kcache = e->kc + l * kv_layer; ra.vcache = e->vc + l * kv_layer;
             ra.pos0 = pos; ra.n_heads = e->n_heads_l; ra.n_kv = e->n_kv_l; ra.hd = p.head_dim; ra.q_dim = qd; ra.kv_dim = kd; ra.max_seq = p.max_seq_len;
             ra.rope_fast = (p.flags & CUQWEN_FLAG_ACCURATE_ROPE) ? 0 : 1; ra.theta = p.rope_theta;
-            PK(launch_pf_rope_kv(ra, T, e->stream));
+            PK(launch_pf_rope_kv(ra, T, cfg));
             if (l == p.n_layers - 1) break;              // the last layer's keys and values are stored: nothing after them feeds the cache
             PfAttnArgs aa; memset(&aa, 0, sizeof aa);
             aa.q = e->pf_q; aa.kc = ra.kcache; aa.vc = ra.vcache; aa.out = e->pf_att; aa.T = T; aa.pos0 = pos; aa.n_heads = e->n_heads_l;
             aa.grp = e->plan.grp; aa.max_seq = p.max_seq_len; aa.ldq = qd; aa.scale_log2 = (1.0f / sqrtf((float)p.head_dim)) * 1.4426950408889634f;
-            if (!(p.flags & CUQWEN_FLAG_PREFILL_ATTN_MMA)) PK(launch_prefill_attn_tc(p.head_dim, aa, e->n_kv_l, t_err, e->stream));
+            if (!(p.flags & CUQWEN_FLAG_PREFILL_ATTN_MMA)) PK(launch_prefill_attn_tc(p.head_dim, aa, e->n_kv_l, t_err, cfg));
             else PK(launch_prefill_attn(p.head_dim, aa, e->stream));
             if (int r = prefill_gemm(e, PF_RESID, e->pf_att, om, 1, e->pf_x, T, p.dim)) return r;
-            PK(launch_pf_rmsnorm(e->pf_x, L.post_norm, e->pf_xn, T, p.dim, eps, e->stream));
+            PK(launch_pf_rmsnorm(e->pf_x, L.post_norm, e->pf_xn, T, p.dim, eps, cfg));
             if (int r = prefill_gemm(e, PF_SWIGLU, e->pf_xn, gu, 2, e->pf_g, T, e->inter_l)) return r;
             if (int r = prefill_gemm(e, PF_RESID, e->pf_g, dm, 1, e->pf_x, T, p.dim)) return r;
         }
@@ -1249,7 +1251,7 @@ extern "C" int cuqwen_k_prefill_attention(int device, int impl, const void* q, c
     a.q = (const __half*)q; a.kc = (const __half*)kcache; a.vc = (const __half*)vcache; a.out = (__half*)out; a.T = n_tokens; a.pos0 = pos0;
     a.n_heads = n_heads; a.grp = n_heads / n_kv_heads; a.max_seq = max_seq_len; a.ldq = q_stride;
     a.scale_log2 = (1.0f / sqrtf((float)head_dim)) * 1.4426950408889634f;
-    if (impl == 0) KK(launch_prefill_attn_tc(head_dim, a, n_kv_heads, t_err, dc->stream));
+    if (impl == 0) KK(launch_prefill_attn_tc(head_dim, a, n_kv_heads, t_err, LaunchCfg{dc->stream, dc->sms, false}));
     else KK(launch_prefill_attn(head_dim, a, dc->stream));
     return CUQWEN_OK;
 }

@@ -60,10 +60,12 @@ __global__ void __launch_bounds__(kLpThreads, 2) latent_prefill_attn_kernel(cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = lds32(tmem_slot);
+    pdl_launch_dependents();      // after the allocation: what the next launch takes early can not keep a CTA of this one waiting
     const uint32_t tS = tmem, tO = tmem + 2u * kLpBN;
 
     if (warp == 0) {
         if (lane == 0) {
+            pdl_wait();
             mbar_expect_tx(b_q, (uint32_t)(nbk * kLpQBlk));
             for (int b = 0; b < a.nbn; ++b) tma_load_3d(sQ + b * kLpQBlk, &a.tqn, 64 * b, head, q0, b_q);
             for (int b = 0; b < a.nbr; ++b) tma_load_3d(sQ + (a.nbn + b) * kLpQBlk, &a.tqr, 64 * b, head, q0, b_q);
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(kLpThreads, 2) latent_prefill_attn_kernel(cons
         if (hsel == 1) l = mxbuf[128 + r];
         if (!failed && !mbar_wait(b_pv, (uint32_t)(nj - 1) & 1u)) failed = true;
         tc_fence_after();
+        pdl_wait();               // the gate is an earlier launch's output
         const float inv = a.out_scale / l;
         const int t = q0 + r;
 #pragma unroll 1

@@ -1,6 +1,7 @@
 // Batched prefill: argument blocks and launchers of the attention and row-wise kernels (prefill_attn.cu); the GEMM is in
 // prefill_gemm.cuh.  The reference prefills one token at a time through the decode path (src/main.cu:86-92).
 #pragma once
+#include "launch.h"
 #include "tma.cuh"
 
 namespace cq {
@@ -15,7 +16,7 @@ struct PfAttnArgs {
 };
 int launch_prefill_attn(int head_dim, const PfAttnArgs& a, cudaStream_t stream);          // mma.sync, head_dim 64 / 128
 // tcgen05 kernel, head_dim 64 / 128; kc / vc must be the caches' [n_kv][max_seq][head_dim] base.  *err receives a code when a bounded wait expires.
-int launch_prefill_attn_tc(int head_dim, const PfAttnArgs& a, int n_kv, unsigned* err, cudaStream_t stream);
+int launch_prefill_attn_tc(int head_dim, const PfAttnArgs& a, int n_kv, unsigned* err, const LaunchCfg& cfg);
 
 struct PfRopeArgs {
     const float* qkv;         // [T][q_dim + 2 kv_dim] fp32 sums
@@ -25,8 +26,8 @@ struct PfRopeArgs {
     int pos0, n_heads, n_kv, hd, q_dim, kv_dim, max_seq, rope_fast;
     float theta;
 };
-int launch_pf_embed(const __half* table, const int* d_tokens, __half* x, int T, int dim, cudaStream_t s);
-int launch_pf_rmsnorm(const __half* x, const __half* w, __half* out, int T, int dim, float eps, cudaStream_t s);
-int launch_pf_rope_kv(const PfRopeArgs& a, int T, cudaStream_t s);
+int launch_pf_embed(const __half* table, const int* d_tokens, __half* x, int T, int dim, const LaunchCfg& cfg);
+int launch_pf_rmsnorm(const __half* x, const __half* w, __half* out, int T, int dim, float eps, const LaunchCfg& cfg);
+int launch_pf_rope_kv(const PfRopeArgs& a, int T, const LaunchCfg& cfg);
 
 }  // namespace cq

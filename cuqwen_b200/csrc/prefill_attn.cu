@@ -9,6 +9,7 @@
 // mma.sync.m16n8k16 with fp32 accumulation and an fp32 online softmax; query t (cache position pos0 + t) sees keys
 // [0, pos0 + t].
 #include "prefill.cuh"
+#include "stack_dev.cuh"
 
 namespace cq {
 
@@ -181,6 +182,7 @@ int launch_prefill_attn(int head_dim, const PfAttnArgs& a, cudaStream_t stream) 
 
 // ---- row-wise kernels -----------------------------------------------------------------------------------------------
 __global__ void pf_embed_kernel(const __half* __restrict__ table, const int* __restrict__ tokens, __half* __restrict__ x, int dim) {
+    pdl_launch_dependents(); pdl_wait();
     const uint4* src = reinterpret_cast<const uint4*>(table + (size_t)tokens[blockIdx.x] * dim);
     uint4* dst = reinterpret_cast<uint4*>(x + (size_t)blockIdx.x * dim);
     for (int i = threadIdx.x; i < dim / 8; i += blockDim.x) dst[i] = src[i];
@@ -189,6 +191,7 @@ __global__ void pf_embed_kernel(const __half* __restrict__ table, const int* __r
 // out[t] = half(x[t] * rsqrt(mean(x[t]^2) + eps) * w), one CTA per token
 __global__ void __launch_bounds__(256) pf_rmsnorm_kernel(const __half* __restrict__ x, const __half* __restrict__ w, __half* __restrict__ out, int dim, float eps) {
     __shared__ float red[33];
+    pdl_launch_dependents(); pdl_wait();
     const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)blockIdx.x * dim);
     uint4* orow = reinterpret_cast<uint4*>(out + (size_t)blockIdx.x * dim);
     const uint4* wr = reinterpret_cast<const uint4*>(w);
@@ -210,6 +213,7 @@ __global__ void __launch_bounds__(256) pf_rmsnorm_kernel(const __half* __restric
 // qkv: fp32 [T][q_dim + 2 kv_dim] straight from the GEMMs.  Bias in fp32, one rounding to fp16, rotate-half RoPE on q
 // and k from the rounded values, k and v into cache row pos0 + t - the arithmetic of the decode kernel's epilogue.
 __global__ void pf_rope_kv_kernel(const PfRopeArgs a) {
+    pdl_launch_dependents(); pdl_wait();
     const int tkn = blockIdx.x, half_hd = a.hd / 2;
     const int nq = a.n_heads * half_hd, nk = a.n_kv * half_hd;
     const float* row = a.qkv + (size_t)tkn * (a.q_dim + 2 * a.kv_dim);
@@ -238,17 +242,14 @@ __global__ void pf_rope_kv_kernel(const PfRopeArgs a) {
     }
 }
 
-int launch_pf_embed(const __half* table, const int* d_tokens, __half* x, int T, int dim, cudaStream_t s) {
-    pf_embed_kernel<<<T, 128, 0, s>>>(table, d_tokens, x, dim);
-    return (int)cudaGetLastError();
+int launch_pf_embed(const __half* table, const int* d_tokens, __half* x, int T, int dim, const LaunchCfg& cfg) {
+    return st_launch(pf_embed_kernel, dim3(T), dim3(128), 0, cfg, table, d_tokens, x, dim);
 }
-int launch_pf_rmsnorm(const __half* x, const __half* w, __half* out, int T, int dim, float eps, cudaStream_t s) {
-    pf_rmsnorm_kernel<<<T, 256, 0, s>>>(x, w, out, dim, eps);
-    return (int)cudaGetLastError();
+int launch_pf_rmsnorm(const __half* x, const __half* w, __half* out, int T, int dim, float eps, const LaunchCfg& cfg) {
+    return st_launch(pf_rmsnorm_kernel, dim3(T), dim3(256), 0, cfg, x, w, out, dim, eps);
 }
-int launch_pf_rope_kv(const PfRopeArgs& a, int T, cudaStream_t s) {
-    pf_rope_kv_kernel<<<T, 256, 0, s>>>(a);
-    return (int)cudaGetLastError();
+int launch_pf_rope_kv(const PfRopeArgs& a, int T, const LaunchCfg& cfg) {
+    return st_launch(pf_rope_kv_kernel, dim3(T), dim3(256), 0, cfg, a);
 }
 
 }  // namespace cq

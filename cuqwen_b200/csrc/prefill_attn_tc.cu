@@ -13,6 +13,7 @@
 // S of the next tile is issued before the current tile's P is waited for, so Q K^T overlaps the softmax.
 // Every mbarrier wait is bounded; a wait that runs out sets *err and the CTA drains.
 #include "prefill.cuh"
+#include "stack_dev.cuh"
 #include "tcgen05.cuh"
 
 namespace cq {
@@ -69,10 +70,12 @@ __global__ void __launch_bounds__(kTaThreads, 2) prefill_attn_tc_kernel(const __
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = lds32(tmem_slot);
+    pdl_launch_dependents();      // after the allocation: what the next launch takes early can not keep a CTA of this one waiting
     const uint32_t tS = tmem, tO = tmem + 2u * kTaBN;
 
     if (warp == 0) {
         if (lane == 0) {
+            pdl_wait();           // everything below follows from these loads
             mbar_expect_tx(b_q, (uint32_t)kTaQTile);
             for (int b = 0; b < NBLK; ++b) tma_load_2d(sQ + b * kTaQHalf, &a.tq, head * kTaHD + 64 * b, q0, b_q);
             for (int j = 0; j < nj; ++j) {
@@ -232,18 +235,17 @@ static TaEncodeFn ta_encode() {
 }
 
 template <int HD>
-static int ta_go(const PfAttnTcArgs& k, dim3 grid, cudaStream_t stream) {
+static int ta_go(const PfAttnTcArgs& k, dim3 grid, const LaunchCfg& cfg) {
     static bool once = false;
     if (!once) {
         const cudaError_t e = cudaFuncSetAttribute(prefill_attn_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ta_smem(HD));
         if (e != cudaSuccess) return (int)e;
         once = true;
     }
-    prefill_attn_tc_kernel<HD><<<grid, kTaThreads, ta_smem(HD), stream>>>(k);
-    return (int)cudaGetLastError();
+    return st_launch(prefill_attn_tc_kernel<HD>, grid, dim3(kTaThreads), (size_t)ta_smem(HD), cfg, k);
 }
 
-int launch_prefill_attn_tc(int head_dim, const PfAttnArgs& a, int n_kv, unsigned* err, cudaStream_t stream) {
+int launch_prefill_attn_tc(int head_dim, const PfAttnArgs& a, int n_kv, unsigned* err, const LaunchCfg& cfg) {
     const int kTaHD = head_dim;
     if (head_dim != 64 && head_dim != 128) return (int)cudaErrorInvalidValue;
     if (a.T <= 0 || a.pos0 < 0 || a.pos0 + a.T > a.max_seq || a.n_heads <= 0 || a.grp <= 0 || a.ldq % 8 || n_kv <= 0) return (int)cudaErrorInvalidValue;
@@ -268,7 +270,7 @@ int launch_prefill_attn_tc(int head_dim, const PfAttnArgs& a, int n_kv, unsigned
     }
     k.out = a.out; k.T = a.T; k.pos0 = a.pos0; k.n_heads = a.n_heads; k.grp = a.grp; k.ldq = a.ldq; k.scale_log2 = a.scale_log2; k.err = err;
     const dim3 grid((a.T + kTaBM - 1) / kTaBM, a.n_heads);
-    return head_dim == 128 ? ta_go<128>(k, grid, stream) : ta_go<64>(k, grid, stream);
+    return head_dim == 128 ? ta_go<128>(k, grid, cfg) : ta_go<64>(k, grid, cfg);
 }
 
 }  // namespace cq

@@ -3,18 +3,25 @@
 // or fp16).  The reference has no such path: it prefills one token at a time through the decode kernels
 // (src/main.cu:86-92; its roadmap names the batched form, README.md:145).
 //
-// One CTA computes a 256-token x NT-row tile as two 128-token halves (one half when the launch has at most 128
-// tokens); NT = 256 weight rows, or 128 / 64 where 256-row tiles would leave most SMs without a CTA.  UMMA shape
-// M = 128 (tokens) x N = NT x K = 16, fp16 operands from shared memory in the K-major 128-byte-swizzled canonical
-// layout, one fp32 accumulator of NT tensor-memory columns per half: the widened weight tile, which costs the CUDA
-// cores more than one half's MMAs cost the tensor core, is used twice.  Per 64-column K block:
-//   warp 0     one lane issues the TMA copies into a ring of three or four slots: the X tiles (128 x 64 fp16,
-//              hardware-swizzled) and the raw weight rows
+// A CTA computes NT weight rows x MH halves of 128 tokens.  UMMA shape M = 128 (tokens) x N = NT x K = 16, fp16 operands from shared
+// memory in the K-major 128-byte-swizzled canonical layout, one fp32 accumulator in tensor memory per half: the
+// widened weight tile, which costs the CUDA cores more than one half's MMAs cost the tensor core, is used by all halves.
+// Per 64-column K block:
+//   warp 0     one lane issues the TMA copies into a ring of slots: the X tiles (128 x 64 fp16, hardware-swizzled) and the raw
+//              weight rows; the first slots' weights before the launch it depends on has ended
 //   warps 2-9  quantised weights: a row (or a half / quarter of one) per thread, fp16(q) * scale into the swizzled B
 //              tile, a ring of two slots (fp16 weights arrive swizzled by TMA and skip this)
 //   warp 1     one lane issues four tcgen05.mma (K = 16 each) per half and commits the slots back to their fillers
+// Two forms of clusters:
+//   pairs (CG = 2)   two CTAs work on one tile of twice the tokens (cta_group::2, M = 256): each keeps half of the weight rows in its
+//              shared memory, so that rows are widened once for 512 tokens.  A single CTA with two halves moves 176 KB through shared
+//              memory per int4 K block, 1375 cycles' worth for 1024 cycles of MMAs; one of a pair 120 KB, 940 cycles' worth.
+//   split (gridDim.z = S)   S CTAs share a tile's K blocks and exchange partial sums through distributed shared memory, each finishing
+//              1 / S of the tile: no sums in global memory, and a fixed order of adding.
 // After the last K block warps 2-9 read the accumulators (tcgen05.ld, warp w owns TMEM lanes 32 * (w % 4) ..) and
-// apply the epilogue.  Every mbarrier wait is bounded (tma.cuh); a wait that runs out sets *err and the CTA drains.
+// apply the epilogue; its loads and stores go through shared memory as whole lines (a token per lane, as tensor memory has it, took
+// 85 us longer for the residual add of 2048 tokens x 3584).  Every mbarrier wait is bounded (tma.cuh); a wait that runs out sets *err and
+// the CTA drains.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -25,19 +32,25 @@ namespace cq {
 constexpr int kPfM = 128;            // tokens per tile
 constexpr int kPfN = 256;            // weight rows per tile at the most (two matrices of half as many rows each in the SwiGLU mode)
 constexpr int kPfKB = 64;            // K per pipeline stage: 128 bytes of fp16, one swizzle row
-constexpr int kPfMH = 2;             // token tiles per CTA: two accumulators share every widened weight tile
 constexpr int kPfConvWarps = 8;      // 8: a weight row of a K block per thread; 16: half a row (measured: no faster, the kernel is bound elsewhere)
 constexpr int kPfThreads = (2 + kPfConvWarps) * 32;
 constexpr int kPfABytes = kPfM * 128;          // one X tile of a stage
-// Shared memory: a ring of NA slots that TMA fills (kPfMH X tiles + the raw weight rows of a K block: int4 32, int8 64
+// Shared memory: a ring of NA slots that TMA fills (MH X tiles + the raw weight rows of a K block: int4 32, int8 64
 // bytes a row) and a ring of NB slots for the fp16 B tile.  The raw data and the X tiles have a TMA round trip to
 // cover, so their ring is the deep one; a widened B tile is consumed by the very next MMAs, two slots suffice.
-// fp16 weights have no raw form: their B tile arrives by TMA, NB = NA.
+// fp16 and bfloat16 weights have no raw form: their B tile arrives by TMA, NB = NA.  The ring takes what an SM has, or half of
+// it for the smallest tile, so that the next launch's first CTAs find room while the last ones of this launch end.
+constexpr int kPfSlack = 1024 /* alignment */ + 512 /* barriers, TMEM address */;
+__host__ __device__ constexpr bool pf_widens(int quant) { return quant == 1 || quant == 2; }
 __host__ __device__ constexpr int pf_raw_bytes(int quant, int nt) { return quant == 2 ? nt * 32 : quant == 1 ? nt * 64 : 0; }
-__host__ __device__ constexpr int pf_na(int quant, int nt = kPfN) { return quant == 3 ? (nt == 256 ? 3 : nt == 128 ? 4 : 5) : quant == 2 ? 4 : 3; }      // bfloat16: narrow tiles leave room for more
-__host__ __device__ constexpr int pf_nb(int quant, int nt = kPfN) { return quant == 3 ? pf_na(3, nt) : quant == 0 ? 3 : 2; }
-__host__ __device__ constexpr int pf_smem_bytes(int quant, int nt) {
-    return pf_na(quant, nt) * (kPfMH * kPfABytes + pf_raw_bytes(quant, nt)) + pf_nb(quant, nt) * nt * 128 + 1024 /* alignment slack */ + 256 /* barriers, TMEM address */;
+__host__ __device__ constexpr int pf_slot(int quant, int nt, int mh) { return mh * kPfABytes + (pf_widens(quant) ? pf_raw_bytes(quant, nt) : nt * 128); }
+__host__ __device__ constexpr int pf_na(int quant, int nt, int mh) {
+    const int room = (nt == 64 ? 112 : 226) * 1024 - kPfSlack - (pf_widens(quant) ? 2 * nt * 128 : 0), n = room / pf_slot(quant, nt, mh);
+    return n > 8 ? 8 : n;
+}
+__host__ __device__ constexpr int pf_nb(int quant, int nt, int mh) { return pf_widens(quant) ? 2 : pf_na(quant, nt, mh); }
+__host__ __device__ constexpr int pf_smem_bytes(int quant, int nt, int mh) {
+    return pf_na(quant, nt, mh) * pf_slot(quant, nt, mh) + (pf_widens(quant) ? 2 * nt * 128 : 0) + kPfSlack;
 }
 
 enum PfMode : int {
@@ -71,8 +84,8 @@ struct PfGemmArgs {
     float* out_f;
     int T, R, K, ldo;          // R: rows of all matrices together; ldo: elements between consecutive tokens of the output
     int mode;
-    int mh;                    // token halves per CTA (1 or 2), set by the launcher
     unsigned* err;
+    int pdl;                   // launch under programmatic dependent launch
     // Q_BF16
     __nv_bfloat16* out_b;
     CUtensorMap tx2, tw2;      // a second product summed into the same rows (K2 = 0: none)

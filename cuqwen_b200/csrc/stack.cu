@@ -556,9 +556,9 @@ int stack_run_chunk(cuqwen_engine* e, int T, int pos0, const int* want, int n_wa
         SK(cudaMalloc((void**)&s->xn_rows, (size_t)kLogitRows * s->wp * s->esz));
         SK(cudaMalloc((void**)&s->want_rows, (size_t)kChunk * 4));
     }
-    const LaunchCfg cfg{e->stream, e->sms, false};
+    const LaunchCfg plain{e->stream, e->sms, false}, cfg{e->stream, e->sms, !(e->p.flags & CUQWEN_FLAG_NO_PDL)};      // plain: launches that follow a copy
     Pass p{e, s, &s->pf, cfg, T, false, e->pf_tok, nullptr, pos0, nullptr};
-    if (int r = p.done(launch_st_embed(s->embed.w, s->embed.pitch, e->pf_tok, s->pf.x, s->wp, s->spec.width, (float)s->spec.embed_scale, T, cfg), "embedding")) return r;
+    if (int r = p.done(launch_st_embed(s->embed.w, s->embed.pitch, e->pf_tok, s->pf.x, s->wp, s->spec.width, (float)s->spec.embed_scale, T, plain), "embedding")) return r;
     if (int r = s->spec.sequential ? p.seq_layers(n_want == 0) : p.layers(n_want == 0)) return r;
     if (n_want == 0) return CUQWEN_OK;
     if (p.last_y()) if (int r = p.norms(p.last_y(), p.last_y_w(), nullptr, nullptr)) return r;
@@ -567,7 +567,7 @@ int stack_run_chunk(cuqwen_engine* e, int T, int pos0, const int* want, int n_wa
         const int n = n_want - i < kLogitRows ? n_want - i : kLogitRows;
         NormRowsArgs a{};
         a.x = s->pf.x; a.ldx = s->wp; a.w[0] = s->final_norm; a.out[0] = s->xn_rows; a.ldo = s->wp; a.n_out = 1; a.width = s->spec.width; a.eps = (float)s->spec.norm_eps; a.rows = s->want_rows + i;
-        if (int r = p.done(launch_st_norms(s->act, a, n, cfg), "final norm")) return r;
+        if (int r = p.done(launch_st_norms(s->act, a, n, plain), "final norm")) return r;
         if (int r = p.head(s->xn_rows, s->logits_rows, n)) return r;
         SK(cudaMemcpy2DAsync(logits_host + (size_t)i * s->spec.vocab, (size_t)s->spec.vocab * 4, s->logits_rows, (size_t)s->vocab_p * 4, (size_t)s->spec.vocab * 4, n, cudaMemcpyDeviceToHost, e->stream));
         SK(cudaStreamSynchronize(e->stream));

@@ -122,7 +122,7 @@ struct Pass {
             PfGemmArgs g; memset(&g, 0, sizeof g);
             PfBf16Mat pm[kPfMaxMat], pm2{};
             for (int i = 0; i < nm; ++i) pm[i] = PfBf16Mat{m[i]->w, m[i]->rows, m[i]->pitch, i * o.var_rows};
-            g.T = n; g.K = pad8(m[0]->cols); g.ldo = ldo; g.out_f = (float*)out; g.out_b = (bf16*)out; g.err = err_word(); g.mode = modes[epi]; g.c0 = o.c0; g.c1 = o.c1; g.bias_f = o.bias;
+            g.T = n; g.K = pad8(m[0]->cols); g.ldo = ldo; g.out_f = (float*)out; g.out_b = (bf16*)out; g.err = err_word(); g.mode = modes[epi]; g.c0 = o.c0; g.c1 = o.c1; g.bias_f = o.bias; g.pdl = cfg.pdl;
             if (o.m2) { pm2 = PfBf16Mat{o.m2->w, o.m2->rows, o.m2->pitch}; g.K2 = o.m2->cols; }
             if (o.side) { g.side = o.side->side; g.side_pitch = o.side->side_pitch; g.side_dim = o.side->side_dim; g.tokens = o.side->tokens; }
             GO(launch_prefill_gemm_bf16(g, x, ldx, pm, nm, o.m2 ? o.x2 : nullptr, o.ldx2, o.m2 ? &pm2 : nullptr, cfg.stream));

@@ -44,6 +44,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         else if (now - t0 > 4000000000ll) return false;
     }
 }
+// Cluster forms: an address of another CTA's shared memory, and an arrival there.  The arrival carries no cluster-wide release (one
+// costs a memory barrier, measured about 1 us): it announces data in the arriving CTA's own shared memory, made visible
+// to the async proxy there before, which that CTA's own tensor core then reads.
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory"); }
+// All threads of all CTAs of the cluster take part.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // global -> shared bulk copy; completion is signalled on `bar` with the byte count.  dst, src and bytes are multiples of 16.
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");

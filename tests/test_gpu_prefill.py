@@ -73,6 +73,36 @@ def test_prefill_gemm_swiglu(built, quant, T, R, Kc):
     assert close(got, want), report(got, want)
 
 
+# Every tile shape and split that the launcher's rule chooses, each at a size with ragged tokens and rows: splits of K over two, four and
+# eight CTAs, pairs of CTAs with 128, 192, 224 and 256 rows, one and two token halves.
+@pytest.mark.parametrize("quant", [2, 1, 0])
+@pytest.mark.parametrize("T,R,Kc", [(1, 72, 640), (5, 72, 2048), (37, 2312, 2048), (61, 6408, 2048), (61, 6408, 3072), (33, 904, 3072), (129, 6408, 256), (257, 6408, 256), (257, 8200, 256),
+                                    (513, 3080, 256), (513, 6408, 256), (513, 8200, 256), (700, 6408, 256), (1025, 6408, 256), (500, 1800, 3072)])
+def test_prefill_gemm_tiles_and_splits(built, quant, T, R, Kc):
+    test_prefill_gemm_plain_modes(built, quant, T, R, Kc)
+
+
+@pytest.mark.parametrize("quant", [2, 1, 0])
+@pytest.mark.parametrize("T,R,Kc", [(1, 72, 640), (61, 1152, 2048), (61, 72, 3072), (61, 3080, 3072), (61, 6408, 3072), (129, 3080, 256), (129, 6408, 256), (129, 8200, 256), (257, 6408, 256),
+                                    (257, 8200, 256), (513, 3080, 256), (700, 3080, 256), (1025, 3080, 256)])
+def test_prefill_gemm_swiglu_tiles_and_splits(built, quant, T, R, Kc):
+    rng = np.random.default_rng(T + R * 3 + quant)
+    x = rng.standard_normal((T, Kc)).astype(np.float16)
+    (wg, sg), (wu, su) = (quant_mats(rng, R, Kc, quant, full_range=False, sigma=0.05) for _ in range(2))
+    dg, du, xf = dequant(wg, sg, quant, Kc), dequant(wu, su, quant, Kc), x.astype(np.float64)
+    g, u = xf @ dg.T, xf @ du.T
+    silu = g / (1.0 + np.exp(-g))
+    out = DevBuf(T * R * 2)
+    K.prefill_gemm(quant, K.PF_SWIGLU, dev(x), dev(wg), dev(sg) if sg is not None else None, out, T, R, Kc, w1=dev(wu), s1=dev(su) if su is not None else None)
+    sync()
+    got = out.numpy(np.float16).reshape(T, R).astype(np.float64)
+    # a widened weight is rounded to fp16 (relative 2^-11 at most, 2^-11 / sqrt(3) rms), so a sum is off by six times that of its terms
+    # together at most; |silu'| <= 1.1; the result is rounded to fp16, after a fast exponential and divide
+    e = [6 * 2.0 ** -11 / 3 ** 0.5 * np.sqrt((xf * xf) @ (d * d).T) for d in (dg, du)]
+    lim = 1.1 * np.abs(u) * e[0] + np.abs(silu) * e[1] + e[0] * e[1] + 2.0 ** -10 * np.abs(silu * u) + 1e-4
+    assert (np.abs(got - silu * u) <= lim).all(), report(got, silu * u)
+
+
 CFGS = {
     "hd128": dict(vocab=2048, dim=512, inter=1280, layers=3, heads=4, kv=2, hd=128, tied=False),
     "hd64": dict(vocab=1024, dim=256, inter=768, layers=4, heads=4, kv=2, hd=64, tied=True),

@@ -84,6 +84,12 @@ def test_linear(built, act, n, rows, cols, cols2):
         near(read_act(out, "float32" if f32 else act, (n, rows)), want, "float32" if f32 else act)
 
 
+# tiles and splits of the tensor-core GEMM that the sizes above do not reach (with and without a second product)
+@pytest.mark.parametrize("n,rows,cols,cols2", [(33, 904, 2048, 1024), (61, 6408, 1000, 520), (129, 6408, 256, 0), (257, 8200, 200, 72), (513, 8200, 256, 0), (700, 6408, 192, 64), (1025, 6408, 256, 0)])
+def test_linear_tiles_and_splits(built, n, rows, cols, cols2):
+    test_linear(built, "bfloat16", n, rows, cols, cols2)
+
+
 @pytest.mark.parametrize("act", ACTS)
 @pytest.mark.parametrize("width", [8, 100, 1536, 3000, 9000])
 def test_norm_rows_and_the_added_token_input(built, act, width):
