@@ -1,6 +1,7 @@
 // Host side of the decode engine: model table, weight loader, state, the
 // per-step launch sequence and its CUDA graph, tensor-parallel plumbing, and
 // the extern "C" boundary declared in include/cuqwen_b200.h.
+#include <algorithm>
 #include <dlfcn.h>
 #include <fcntl.h>
 #include <nccl.h>
@@ -687,8 +688,25 @@ extern "C" int cuqwen_step(cuqwen_engine* e, int token, int pos, const int* hist
 // batched prefill: the prompt's tokens go through every layer as tiles, the KV cache rows [pos0, pos0 + n) come out.
 // The reference runs qwen_forward once per prompt token for the same effect (src/main.cu:86-92).
 // ---------------------------------------------------------------------------
-constexpr int kPrefillChunk = 2048;
+// Tokens that go through the layers together.  Long enough that a projection of few rows fills several waves of SMs (14B, o_proj
+// and down: 2048 tokens are 92 pair tiles for 74 pairs of SMs, two waves for 1.24; 8192 are 368, five for 4.97), short enough
+// that the workspace stays below 1 GB (14B: 96 KB a token).
+constexpr int kPrefillChunk = 8192;
 #define PK(call) do { int r_ = (call); if (r_) return fail(r_ == (int)cudaErrorInvalidValue ? CUQWEN_ERR_ARG : CUQWEN_ERR_CUDA, "%s: %s", #call, cudaGetErrorString((cudaError_t)r_)); } while (0)
+
+// The workspace holds as many tokens as the longest portion so far, rounded up; a portion beyond it gets a new one of at least twice the size.
+static int prefill_workspace(cuqwen_engine* e, int need) {
+    if (need <= e->pf_rows) return CUQWEN_OK;
+    const cuqwen_params& p = e->p;
+    const size_t C = (size_t)std::min(kPrefillChunk, std::max((need + 255) / 256 * 256, 2 * e->pf_rows)), qd = (size_t)e->q_dim_l, kd = (size_t)e->kv_dim_l;
+    struct { void** at; size_t bytes; } const bufs[] = {{(void**)&e->pf_x, C * p.dim * 2}, {(void**)&e->pf_xn, C * p.dim * 2}, {(void**)&e->pf_qkv, C * (qd + 2 * kd) * 4}, {(void**)&e->pf_q, C * qd * 2},
+                                                        {(void**)&e->pf_att, C * qd * 2}, {(void**)&e->pf_g, C * e->inter_l * 2}, {(void**)&e->pf_tok, C * 4}};
+    e->pf_rows = 0;
+    for (const auto& b : bufs) { if (*b.at) cudaFree(*b.at); *b.at = nullptr; }      // no portion is in flight: every call ends with a synchronisation
+    for (const auto& b : bufs) CK(cudaMalloc(b.at, b.bytes));
+    e->pf_rows = (int)C;
+    return CUQWEN_OK;
+}
 
 static int prefill_gemm(cuqwen_engine* e, int mode, const __half* x, const Mat* const* mats, int nmat, void* out, int T, int ldo) {
     PfGemmArgs a; memset(&a, 0, sizeof a);
@@ -710,6 +728,7 @@ static int check_tokens(const cuqwen_engine* e, const int* tokens, int n_tokens,
 static int stack_portion(cuqwen_engine* e, const int* tokens, int n_tokens, int pos0, const int* want, int n_want, float* logits) {
     const int C = stack_chunk();
     CK(cudaSetDevice(e->p.device));
+    if (int r = stack_workspace(e->stack, std::min(n_tokens, C))) return r;
     if (int r = stack_begin(e->stack, pos0)) return r;
     t_err = reinterpret_cast<unsigned*>(&e->ctl->pad[0]);
     if (!e->pf_tok) CK(cudaMalloc((void**)&e->pf_tok, (size_t)C * 4));
@@ -780,12 +799,7 @@ extern "C" int cuqwen_prefill(cuqwen_engine* e, const int* tokens, int n_tokens,
     CK(cudaSetDevice(p.device));
     t_err = reinterpret_cast<unsigned*>(&e->ctl->pad[0]);
     const int qd = e->q_dim_l, kd = e->kv_dim_l, C = kPrefillChunk;
-    if (!e->pf_x) {
-        CK(cudaMalloc((void**)&e->pf_x, (size_t)C * p.dim * 2)); CK(cudaMalloc((void**)&e->pf_xn, (size_t)C * p.dim * 2));
-        CK(cudaMalloc((void**)&e->pf_qkv, (size_t)C * (qd + 2 * kd) * 4)); CK(cudaMalloc((void**)&e->pf_q, (size_t)C * qd * 2));
-        CK(cudaMalloc((void**)&e->pf_att, (size_t)C * qd * 2)); CK(cudaMalloc((void**)&e->pf_g, (size_t)C * e->inter_l * 2));
-        CK(cudaMalloc((void**)&e->pf_tok, (size_t)C * 4));
-    }
+    if (int r = prefill_workspace(e, std::min(n_tokens, C))) return r;
     const size_t kv_layer = (size_t)e->n_kv_l * p.max_seq_len * p.head_dim;
     const float eps = __half2float(__float2half(p.norm_eps));
     const int ldqkv = qd + 2 * kd;

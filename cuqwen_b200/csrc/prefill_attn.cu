@@ -212,33 +212,41 @@ __global__ void __launch_bounds__(256) pf_rmsnorm_kernel(const __half* __restric
 
 // qkv: fp32 [T][q_dim + 2 kv_dim] straight from the GEMMs.  Bias in fp32, one rounding to fp16, rotate-half RoPE on q
 // and k from the rounded values, k and v into cache row pos0 + t - the arithmetic of the decode kernel's epilogue.
-__global__ void pf_rope_kv_kernel(const PfRopeArgs a) {
-    pdl_launch_dependents(); pdl_wait();
-    const int tkn = blockIdx.x, half_hd = a.hd / 2;
-    const int nq = a.n_heads * half_hd, nk = a.n_kv * half_hd;
-    const float* row = a.qkv + (size_t)tkn * (a.q_dim + 2 * a.kv_dim);
+// CTA = token.  Bound by memory (six bytes a value): the hd / 2 angles are the same for all heads and computed once, and a thread
+// takes four neighbouring pairs of a head, so that its loads are 16 bytes and its stores 8.
+constexpr int kPfRopeMaxHalf = 64;            // head_dim up to 128, as cuqwen_prefill takes
+__global__ void __launch_bounds__(256) pf_rope_kv_kernel(const PfRopeArgs a) {
+    __shared__ __align__(16) float cs[2][kPfRopeMaxHalf];
+    pdl_launch_dependents();
+    const int tkn = blockIdx.x, half_hd = a.hd / 2, per_head = half_hd / 4;
     const int pos = a.pos0 + tkn;
-    for (int i = threadIdx.x; i < nq + 2 * nk; i += blockDim.x) {
-        const int mat = i < nq ? 0 : i < nq + nk ? 1 : 2;
-        const int j = mat == 0 ? i : mat == 1 ? i - nq : i - nq - nk;
-        const int head = j / half_hd, d = j % half_hd;
-        const int ra = head * a.hd + d, rb = ra + half_hd;
-        const int off = mat == 0 ? 0 : mat == 1 ? a.q_dim : a.q_dim + a.kv_dim;
+    if (threadIdx.x < half_hd) rope_cs(threadIdx.x, a.hd, pos, a.theta, a.rope_fast, &cs[0][threadIdx.x], &cs[1][threadIdx.x]);
+    pdl_wait();
+    __syncthreads();
+    const float* row = a.qkv + (size_t)tkn * (a.q_dim + 2 * a.kv_dim);
+    for (int i = threadIdx.x; i < (a.n_heads + 2 * a.n_kv) * per_head; i += 256) {
+        int head = i / per_head;
+        const int d = (i - head * per_head) * 4, mat = head < a.n_heads ? 0 : head < a.n_heads + a.n_kv ? 1 : 2;
+        const float* src = row + head * a.hd + d;             // the three matrices' columns lie side by side
+        head -= mat == 0 ? 0 : mat == 1 ? a.n_heads : a.n_heads + a.n_kv;
         const __half* bias = mat == 0 ? a.bq : mat == 1 ? a.bk : a.bv;
-        const float b0 = bias ? __half2float(bias[ra]) : 0.f, b1 = bias ? __half2float(bias[rb]) : 0.f;
-        const float f0 = __half2float(__float2half(row[off + ra] + b0)), f1 = __half2float(__float2half(row[off + rb] + b1));
-        __half o0, o1;
-        if (mat < 2) {
-            float c, s;
-            rope_cs(d, a.hd, pos, a.theta, a.rope_fast, &c, &s);
-            o0 = __float2half(f0 * c - f1 * s); o1 = __float2half(f1 * c + f0 * s);
-        } else { o0 = __float2half(f0); o1 = __float2half(f1); }
-        if (mat == 0) { a.q_out[(size_t)tkn * a.q_dim + ra] = o0; a.q_out[(size_t)tkn * a.q_dim + rb] = o1; }
-        else {
-            __half* cache = mat == 1 ? a.kcache : a.vcache;
-            const size_t base = ((size_t)head * a.max_seq + pos) * a.hd;
-            cache[base + d] = o0; cache[base + d + half_hd] = o1;
+        const float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + half_hd);
+        float f0[4] = {lo.x, lo.y, lo.z, lo.w}, f1[4] = {hi.x, hi.y, hi.z, hi.w};
+        __align__(8) __half o0[4], o1[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int ra = head * a.hd + d + k;
+            const float b0 = bias ? __half2float(bias[ra]) : 0.f, b1 = bias ? __half2float(bias[ra + half_hd]) : 0.f;
+            f0[k] = __half2float(__float2half(f0[k] + b0)); f1[k] = __half2float(__float2half(f1[k] + b1));
+            if (mat < 2) {
+                const float c = cs[0][d + k], s = cs[1][d + k];
+                o0[k] = __float2half(f0[k] * c - f1[k] * s); o1[k] = __float2half(f1[k] * c + f0[k] * s);
+            } else { o0[k] = __float2half(f0[k]); o1[k] = __float2half(f1[k]); }
         }
+        __half* cache = mat == 1 ? a.kcache : a.vcache;
+        __half* dst = (mat == 0 ? a.q_out + (size_t)tkn * a.q_dim + head * a.hd : cache + ((size_t)head * a.max_seq + pos) * a.hd) + d;
+        *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o0);
+        *reinterpret_cast<uint2*>(dst + half_hd) = *reinterpret_cast<const uint2*>(o1);
     }
 }
 

@@ -547,15 +547,23 @@ int stack_record_step(cuqwen_engine* e, const LaunchCfg& cfg, const std::functio
     return p.head(s->dec.xn1, s->logits, 1);
 }
 
+// Workspace of a portion: rows for the longest so far, at least twice as many when it has to grow.  No portion is in flight here.
+int stack_workspace(Stack* s, int need) {
+    if (!s->logits_rows) {
+        if (!s->xn_rows) SK(cudaMalloc((void**)&s->xn_rows, (size_t)kLogitRows * s->wp * s->esz));
+        if (!s->want_rows) SK(cudaMalloc((void**)&s->want_rows, (size_t)kChunk * 4));
+        SK(cudaMalloc((void**)&s->logits_rows, (size_t)kLogitRows * s->vocab_p * 4));
+    }
+    if (need <= s->pf.rows) return CUQWEN_OK;
+    const int most = kChunk < s->max_seq ? kChunk : s->max_seq, rows = (need + 255) / 256 * 256, twice = 2 * s->pf.rows, want = rows > twice ? rows : twice;
+    if (s->pf.arena) SK(cudaFree(s->pf.arena));
+    s->pf = Stack::Ws{};
+    return alloc_ws(s, &s->pf, want < most ? want : most, false);
+}
+
 int stack_run_chunk(cuqwen_engine* e, int T, int pos0, const int* want, int n_want, float* logits_host) {
     Stack* s = e->stack;
     if (T < 1 || T > kChunk) return report_error(CUQWEN_ERR_ARG, "a portion has 1 to %d tokens", kChunk);
-    if (!s->pf.arena) {
-        if (int r = alloc_ws(s, &s->pf, kChunk < s->max_seq ? kChunk : s->max_seq, false)) return r;
-        SK(cudaMalloc((void**)&s->logits_rows, (size_t)kLogitRows * s->vocab_p * 4));
-        SK(cudaMalloc((void**)&s->xn_rows, (size_t)kLogitRows * s->wp * s->esz));
-        SK(cudaMalloc((void**)&s->want_rows, (size_t)kChunk * 4));
-    }
     const LaunchCfg plain{e->stream, e->sms, false}, cfg{e->stream, e->sms, !(e->p.flags & CUQWEN_FLAG_NO_PDL)};      // plain: launches that follow a copy
     Pass p{e, s, &s->pf, cfg, T, false, e->pf_tok, nullptr, pos0, nullptr};
     if (int r = p.done(launch_st_embed(s->embed.w, s->embed.pitch, e->pf_tok, s->pf.x, s->wp, s->spec.width, (float)s->spec.embed_scale, T, plain), "embedding")) return r;

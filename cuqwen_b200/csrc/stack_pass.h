@@ -13,7 +13,7 @@
 namespace cq {
 
 inline int pad8(int v) { return (v + 7) / 8 * 8; }
-constexpr int kChunk = 2048;                // tokens of a portion that go through the layers together
+constexpr int kChunk = 4096;                // tokens of a portion that go through the layers together (at 7b sizes about 1.2 GB of workspace)
 constexpr int kLogitRows = 64;              // rows of logits computed at a time
 
 struct StMat { bf16* w = nullptr; int rows = 0, cols = 0, pitch = 0; };     // rows with padding, cols with padding of groups
@@ -55,7 +55,7 @@ struct Stack {
     // cache and rotation tables
     uint8_t* cache = nullptr; size_t cache_bytes = 0; std::vector<size_t> cache_off;
     std::vector<RotarySpec> rots; std::vector<float2*> rot_tables;
-    // workspace: a decode step's (one row), and a portion's (kChunk rows; allocated at first use)
+    // workspace: a decode step's (one row), and a portion's (as many rows as the longest so far; stack_workspace)
     struct Ws {
         int rows = 0, kv_rows = 0;
         float *x = nullptr, *x2 = nullptr, *raw = nullptr, *qf = nullptr, *y = nullptr, *o_lat = nullptr, *part_o = nullptr, *part_ml = nullptr;

@@ -264,6 +264,36 @@ def test_prefill_longer_than_one_chunk_and_single_token(built, tmp_path):
     a.close(); b.close()
 
 
+def test_prefill_workspace_grows_and_long_prompts_are_cut(built, tmp_path):
+    """Prompts of 5, 700 and 8192 + 77 tokens through one engine (the workspace grows twice, the last one is cut), each against an engine
+    that is given the same tokens in portions of at most 256."""
+    from cuqwen_b200 import engine as E
+    cfg = dict(vocab=512, dim=256, inter=512, layers=2, heads=2, kv=1, hd=128, tied=True)
+    path = tmp_path / "m.bin"
+    binfmt.write_model(path, cfg, 2, binfmt.random_tensors(cfg, 3))
+    max_seq = 8192 + 128
+    a, b = (E.Engine(E.custom_params(cfg["vocab"], cfg["dim"], cfg["inter"], cfg["layers"], cfg["heads"], cfg["kv"], cfg["hd"], 2, max_seq_len=max_seq)) for _ in range(2))
+    for e in (a, b):
+        e.load(str(path))
+    rng = np.random.default_rng(2)
+    shape = (cfg["layers"], cfg["kv"], max_seq, cfg["hd"])
+    for n in (5, 700, 8192 + 77, 3):
+        toks = rng.integers(0, cfg["vocab"], size=n + 1).astype(np.int32)
+        a.prefill(toks[:n], 0)
+        for i in range(0, n, 256):
+            b.prefill(toks[i:min(n, i + 256)], i)
+        for which in ("KEY_CACHE", "VALUE_CACHE"):
+            ca, cb = (e.read(which).reshape(shape).astype(np.float64)[:, :, :n] for e in (a, b))
+            for part in (slice(0, n), slice(max(0, n - 77), n)):
+                d, r = (ca - cb)[:, :, part], cb[:, :, part]
+                assert np.sqrt((d ** 2).mean()) < 5e-3 * np.sqrt((r ** 2).mean()), f"{which}, {n} tokens"
+        for e in (a, b):
+            e.step(int(toks[n]), n)
+        la, lb = (e.read("LOGITS").astype(np.float64) for e in (a, b))
+        assert np.sqrt(((la - lb) ** 2).mean()) < 1.5e-2 * np.sqrt((lb ** 2).mean()), f"logits, {n} tokens"
+    a.close(); b.close()
+
+
 def attn_oracle(q, Kc, Vc, pos0, nh, nkv, hd):
     """float64 causal attention: q [T][nh*hd], caches [nkv][max_seq][hd]; query t sees keys [0, pos0 + t]."""
     T = q.shape[0]

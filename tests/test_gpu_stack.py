@@ -323,6 +323,19 @@ def test_portions_longer_than_a_chunk(models):
     eng.close()
 
 
+def test_portions_beyond_4096_tokens(models):
+    """The border at which a portion is cut, and a workspace that grows on the way there."""
+    d, cfg, wf, _, _ = models("small")
+    n = 4160
+    toks = np.random.default_rng(5).integers(0, cfg["vocab"], n)
+    eng = E.Engine.open(d, max_seq_len=n)
+    eng.extend(toks[:300], 0, [299])
+    places = [4000, 4094, 4095, 4096, 4097, 4103, 4159]
+    got = eng.extend(toks, 0, places)
+    check(got, np.concatenate([L.forward(cfg, wf, toks[p - 40:p + 1])[-1:] for p in places]), "bfloat16", 1.5)
+    eng.close()
+
+
 @pytest.mark.parametrize("act", ACTS)
 def test_generation_through_step_decode_and_command_line(models, act):
     d, cfg, wf, _, _ = models("small")
