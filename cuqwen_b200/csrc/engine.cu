@@ -451,7 +451,7 @@ static void describe_step(cuqwen_engine* e, std::vector<HostPhase>& out, int nsp
     // SwiGLU output handed to the down projection in staged form: only when the gate/up launch will work on whole
     // 128-row groups, which the launcher decides from the row count
     const bool hand_over = p.quant != 0 && !(p.flags & CUQWEN_FLAG_NO_HANDOVER) && e->inter_l % 128 == 0 &&
-                           gemv_block_rows(e->inter_l, p.dim, e->sms, EPI_SWIGLU) == 128;
+                           gemv_block_rows(e->inter_l, p.dim, e->sms, EPI_SWIGLU, p.quant) == 128;
     // attention output handed to o_proj in staged form: a head of 128 values is one scale group
     const bool att_hand_over = p.quant != 0 && p.head_dim == 128 && !(p.flags & CUQWEN_FLAG_NO_HANDOVER);
     __half* cur = e->x;

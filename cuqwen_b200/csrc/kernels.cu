@@ -482,18 +482,30 @@ static int encode_weight_map(CUtensorMap* m, const void* w, size_t row_bytes, si
 
 constexpr int kGemvThreadsHost = (kConsumerWarps + 1) * 32;
 
-// Rows per CTA block: whole 16-row tiles, as many per block (1, 2, 4 or 8) as keep at least one block per SM.
-// (The kernel takes any row count per block.  Cutting the matrix into SM-count nearly equal blocks instead - 26 rows
-// for the 3584-row projections of the 7B model, 138 blocks in one round where whole tiles give 224 - measured slower:
-// down projection 11.8 against 10.4 us in the step, o_proj 5.9 against 5.1.  The 224 blocks of 16 rows run two to an
-// SM, sixteen consumer warps per SM, and the SMs with one block leave their share of the bandwidth to the others.)
-int gemv_block_rows(int rows, int K, int sm_count, int epi) {
+// Rows per CTA block.  First whole 16-row tiles, as many (1, 2, 4 or 8) as keep at least one block per SM.  int4 matrices of one kind
+// stay there, two blocks to an SM: cutting them into SM-count nearly equal blocks instead (26 rows for the 3584-row projections of the 7B
+// model, 138 blocks where whole tiles give 224) measured slower, down 11.8 against 10.4 us in the step, o_proj 5.9 against
+// 5.1: sixteen consumer warps per SM, and the SMs with one block leave their share of the bandwidth to the others.
+// Everywhere else an SM holds one CTA (its shared memory, or the registers of a two-matrix kernel), blocks go round by round, and a last round
+// that is nearly empty lasts as long as a full one: 4864 rows as 152 blocks of 32 on 148 SMs took a second round for four of them.
+// There the block may have any multiple of eight rows (the scales of a block begin on 16 bytes), if that shortens rounds x rows by a
+// twentieth or more; a block of fewer rows than its row-warps cover idles some of the eight warps.  (Step of the 0.5B int4 model 722 -> 679 us,
+// of six 14B int8 layers 721 -> 685 us.  With many rounds the SMs that are ahead take the memory's rate over: lm_head, nine
+// rounds of 128 rows, was 3 to 7 % slower as nine of 120.)
+int gemv_block_rows(int rows, int K, int sm_count, int epi, int quant) {
     (void)K;
     if (epi == EPI_QKV) return 16;
     const int nsets = (rows + 15) / 16;
     int rw = 1;
     while (rw < 8 && nsets / (rw * 2) >= sm_count) rw *= 2;
-    return 16 * rw;
+    const int whole = 16 * rw;
+    if (sm_count <= 0 || (quant == Q_I4 && epi != EPI_SWIGLU)) return whole;
+    auto rounds = [&](int b) { return ((rows + b - 1) / b + sm_count - 1) / sm_count; };
+    if (rounds(whole) > 3) return whole;
+    int best = whole, cost = rounds(whole) * whole;
+    for (int b = 128; b > whole / 2 && b >= 24; b -= 8)
+        if (20 * rounds(b) * b <= 19 * cost && (best == whole || rounds(b) * b < rounds(best) * best)) best = b;
+    return best;
 }
 
 // Picks the work split (rw row-warps x kw K-parts), the staged piece size and the ring depth for one GEMV launch.
@@ -509,7 +521,7 @@ int launch_gemv(int quant, int epi, GemvArgs& a, const LaunchCfg& cfg) {
     } else {
         if (a.rows <= 0) return (int)cudaErrorInvalidValue;
         a.nsets = (a.rows + 15) / 16;
-        a.brows = gemv_block_rows(a.rows, a.K, cfg.sm_count, epi);
+        a.brows = gemv_block_rows(a.rows, a.K, cfg.sm_count, epi, quant);
         a.nblk = (a.rows + a.brows - 1) / a.brows;
     }
     const int MT = (epi == EPI_SWIGLU || epi == EPI_QKV) ? 2 : 1;
@@ -529,7 +541,7 @@ int launch_gemv(int quant, int epi, GemvArgs& a, const LaunchCfg& cfg) {
     // (CTAs of two consecutive kernels of the step do not share an SM at these register counts.  Capped at 80
     // registers they do, and the step was slower - 574 against 703 tok/s on the 7B int4 model: the early weight
     // copies of the next kernel compete with the loads the running kernel is waiting for.)
-    const int cap_kb = (nblk > cfg.sm_count && quant == Q_I4) ? 110 : 220;
+    const int cap_kb = (nblk > cfg.sm_count && quant == Q_I4 && MT == 1) ? 110 : 220;
     const int per_sm = cap_kb == 110 ? 2 : 1;
     const int grid = nblk < per_sm * cfg.sm_count ? nblk : per_sm * cfg.sm_count;
     const int nsb = nblk <= grid ? 1 : 2;            // a second scale block only when some CTA has a second block

@@ -46,7 +46,7 @@ struct LaunchCfg {
 // size and the ring depth, builds the tensor maps and launches.  Returns a cudaError_t value.
 int launch_gemv(int quant, int epi, GemvArgs& a, const LaunchCfg& cfg);
 // Rows per CTA block that launch_gemv will choose for a matrix of `rows` rows and K input columns.
-int gemv_block_rows(int rows, int K, int sm_count, int epi);
+int gemv_block_rows(int rows, int K, int sm_count, int epi, int quant);
 
 // Byte-typed 3-D tensor map of a row-major matrix seen as [rows][64-byte chunks]: a box of box_rows rows x piece_bytes
 // lands in shared memory chunk-major, [chunk][row][64 bytes].

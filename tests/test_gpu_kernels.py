@@ -143,6 +143,14 @@ def test_gate_up_swiglu(built, quant, dim, inter):
         assert close(got, r), report(got, r)
 
 
+# row counts whose blocks are not whole powers of two of 16-row tiles (40, 80 and 96 rows; the last block a part of one), and their neighbours
+@pytest.mark.parametrize("quant", [0, 1, 2])
+@pytest.mark.parametrize("rows", [4856, 4864, 4880, 5120, 5128, 11008, 13824, 13832])
+def test_blocks_of_any_multiple_of_eight_rows(built, quant, rows):
+    test_gate_up_swiglu(built, quant, 384, rows)
+    test_gemv_add_residual(built, quant, rows, 384)
+
+
 # ---------------------------------------------------------------------------------------------------------------------
 def qkv_inputs(rng, quant, dim, nh, nkv, hd):
     ws = [quant_mats(rng, r, dim, quant, full_range=False) for r in (nh * hd, nkv * hd, nkv * hd)]
