@@ -205,10 +205,8 @@ __device__ __forceinline__ void gemv_consume(const GemvArgs& a, RingCtx& R, int 
 #pragma unroll
                         for (int m = 0; m < MT; ++m) {
                             // columns 0 and 1 (lanes with t == 0) hold sum q*d0 and sum q*d1
-                            const int v0 = (ci[m][0][0] + ci[m][1][0]) + ((ci[m][0][1] + ci[m][1][1]) << 8) - cr;
-                            const int v1 = (ci[m][0][2] + ci[m][1][2]) + ((ci[m][0][3] + ci[m][1][3]) << 8) - cr;
-                            tot[m][0] = fmaf((float)v0, sc[m][0], tot[m][0]);
-                            tot[m][1] = fmaf((float)v1, sc[m][1], tot[m][1]);
+                            tot[m][0] = fmaf((float)(group_sum<Q>(ci[m], 0) - cr), sc[m][0], tot[m][0]);
+                            tot[m][1] = fmaf((float)(group_sum<Q>(ci[m], 2) - cr), sc[m][1], tot[m][1]);
                         }
                     }
                 } else {
