@@ -825,8 +825,9 @@ extern "C" int cuqwen_prefill(cuqwen_engine* e, const int* tokens, int n_tokens,
             PfAttnArgs aa; memset(&aa, 0, sizeof aa);
             aa.q = e->pf_q; aa.kc = ra.kcache; aa.vc = ra.vcache; aa.out = e->pf_att; aa.T = T; aa.pos0 = pos; aa.n_heads = e->n_heads_l;
             aa.grp = e->plan.grp; aa.max_seq = p.max_seq_len; aa.ldq = qd; aa.scale_log2 = (1.0f / sqrtf((float)p.head_dim)) * 1.4426950408889634f;
-            if (!(p.flags & CUQWEN_FLAG_PREFILL_ATTN_MMA)) PK(launch_prefill_attn_tc(p.head_dim, aa, e->n_kv_l, t_err, cfg));
-            else PK(launch_prefill_attn(p.head_dim, aa, e->stream));
+            const bool few = T <= 64 && pos + T <= 256;       // one tile of the mma.sync kernel: its first result is there sooner
+            if (!few && !(p.flags & CUQWEN_FLAG_PREFILL_ATTN_MMA)) PK(launch_prefill_attn_tc(p.head_dim, aa, e->n_kv_l, t_err, cfg));
+            else PK(launch_prefill_attn(p.head_dim, aa, cfg));
             if (int r = prefill_gemm(e, PF_RESID, e->pf_att, om, 1, e->pf_x, T, p.dim)) return r;
             PK(launch_pf_rmsnorm(e->pf_x, L.post_norm, e->pf_xn, T, p.dim, eps, cfg));
             if (int r = prefill_gemm(e, PF_SWIGLU, e->pf_xn, gu, 2, e->pf_g, T, e->inter_l)) return r;
@@ -1266,7 +1267,7 @@ extern "C" int cuqwen_k_prefill_attention(int device, int impl, const void* q, c
     a.n_heads = n_heads; a.grp = n_heads / n_kv_heads; a.max_seq = max_seq_len; a.ldq = q_stride;
     a.scale_log2 = (1.0f / sqrtf((float)head_dim)) * 1.4426950408889634f;
     if (impl == 0) KK(launch_prefill_attn_tc(head_dim, a, n_kv_heads, t_err, LaunchCfg{dc->stream, dc->sms, false}));
-    else KK(launch_prefill_attn(head_dim, a, dc->stream));
+    else KK(launch_prefill_attn(head_dim, a, LaunchCfg{dc->stream, dc->sms, false}));
     return CUQWEN_OK;
 }
 extern "C" int cuqwen_k_gemv_add(int device, int quant, const void* w, const void* s, const void* in, void* x, int rows, int cols) {

@@ -14,7 +14,7 @@ struct PfAttnArgs {
     int T, pos0, n_heads, grp, max_seq, ldq;      // grp = query heads per KV head
     float scale_log2;         // log2(e) / sqrt(hd)
 };
-int launch_prefill_attn(int head_dim, const PfAttnArgs& a, cudaStream_t stream);          // mma.sync, head_dim 64 / 128
+int launch_prefill_attn(int head_dim, const PfAttnArgs& a, const LaunchCfg& cfg);          // mma.sync, head_dim 64 / 128
 // tcgen05 kernel, head_dim 64 / 128; kc / vc must be the caches' [n_kv][max_seq][head_dim] base.  *err receives a code when a bounded wait expires.
 int launch_prefill_attn_tc(int head_dim, const PfAttnArgs& a, int n_kv, unsigned* err, const LaunchCfg& cfg);
 

@@ -51,6 +51,7 @@ template <int HD>
 __global__ void __launch_bounds__(kPaThreads) prefill_attn_kernel(const PfAttnArgs a) {
     constexpr int NCH = HD / 8, KS = HD / 16, TILE = kPaBN * HD * 2;
     extern __shared__ __align__(128) unsigned char pa_smem[];
+    pdl_launch_dependents(); pdl_wait();
     const uint32_t sq = smem_u32(pa_smem), sk = sq + TILE, sv = sk + 2 * TILE;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int head = blockIdx.y, kvh = head / a.grp;
@@ -164,20 +165,20 @@ __global__ void __launch_bounds__(kPaThreads) prefill_attn_kernel(const PfAttnAr
     }
 }
 
-int launch_prefill_attn(int head_dim, const PfAttnArgs& a, cudaStream_t stream) {
+int launch_prefill_attn(int head_dim, const PfAttnArgs& a, const LaunchCfg& cfg) {
     if (a.T <= 0 || a.pos0 < 0 || a.pos0 + a.T > a.max_seq || a.n_heads <= 0 || a.grp <= 0 || a.ldq % 8) return (int)cudaErrorInvalidValue;
     const dim3 grid((a.T + kPaBM - 1) / kPaBM, a.n_heads);
     const size_t smem = (size_t)5 * kPaBN * head_dim * 2;
     if (head_dim == 128) {
         static bool once = false;
         if (!once) { const cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); if (e != cudaSuccess) return (int)e; once = true; }
-        prefill_attn_kernel<128><<<grid, kPaThreads, smem, stream>>>(a);
+        return st_launch(prefill_attn_kernel<128>, grid, dim3(kPaThreads), smem, cfg, a);
     } else if (head_dim == 64) {
         static bool once = false;
         if (!once) { const cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); if (e != cudaSuccess) return (int)e; once = true; }
-        prefill_attn_kernel<64><<<grid, kPaThreads, smem, stream>>>(a);
-    } else return (int)cudaErrorInvalidValue;
-    return (int)cudaGetLastError();
+        return st_launch(prefill_attn_kernel<64>, grid, dim3(kPaThreads), smem, cfg, a);
+    }
+    return (int)cudaErrorInvalidValue;
 }
 
 // ---- row-wise kernels -----------------------------------------------------------------------------------------------

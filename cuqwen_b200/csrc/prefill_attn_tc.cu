@@ -1,16 +1,18 @@
 // Causal attention for a tile of prompt tokens on the tcgen05 tensor cores (head_dim 64 or 128): the batched counterpart of
 // the reference's decode attention (src/kernels.cu:105-288), which the reference applies once per prompt token
-// (src/main.cu:86-92).  prefill_attn.cu holds the mma.sync kernel this one replaces (kept as the comparison variant).
+// (src/main.cu:86-92).  prefill_attn.cu holds an mma.sync kernel for comparison.
 //
-// One CTA = 128 queries of one head, two CTAs to an SM.  Per tile of 64 keys:
-//   warp 0      TMA: K and V tiles of the head's KV group (two 64-column boxes each, hardware-swizzled), two slots
-//   warp 1      one lane issues S = Q K^T (eight MMAs 128 x 64 x 16, both operands K-major) into one of two TMEM
-//               buffers, and - once the softmax warps have written P - O += P V (four MMAs 128 x 128 x 16, V as the MN-major B
-//               operand straight from its cache layout) into a third
-//   warps 2-9   two threads per query row (TMEM lane = row), 32 of the tile's keys each: read S, scale, mask, write
-//               P = 2^(s - m) as fp16 into the swizzled A tile, row sums in fp32; when a row's maximum outgrows m by
-//               2^8, m moves and O is rescaled in TMEM by 2^(m_old - m_new) (rare after the first tiles)
-// S of the next tile is issued before the current tile's P is waited for, so Q K^T overlaps the softmax.
+// One CTA = two tiles of 128 queries of one head, one CTA to an SM.  Per tile of 128 keys:
+//   warp 8      TMA: K and V tiles of the head's KV group (64-column boxes, hardware-swizzled), two slots each
+//   warp 9      one lane issues, for the two query tiles in turn, O += P V of a key tile (A = P from tensor memory, B = V as the MN-major
+//               operand straight from its cache layout) and S = Q K^T of the next (both operands K-major)
+//   warps 0-3   softmax of the first query tile, warps 4-7 of the second: one thread per query row (TMEM lane = row) reads its 128 scores,
+//               masks, writes P = 2^(s - m) as fp16 over them, row sum in fp32; when a row's maximum outgrows m by 2^8, m moves
+//               and O is rescaled in TMEM by 2^(m_old - m_new) (rare after the first tiles)
+// While one tile's softmax runs, the tensor core works for the other.  A row belongs to one thread and P stays in tensor memory, so a tile costs
+// no barrier among the softmax warps and no pass through shared memory; what bounds it is the chain of a tile - scores, exponentials (1024
+// cycles of an SM partition's unit), P V, next scores - of which the two query tiles hide half.
+// The tensor core finishes its MMAs in the order of issue: when S of a key tile is there, so is P V of the one before, and O may be rescaled.
 // Every mbarrier wait is bounded; a wait that runs out sets *err and the CTA drains.
 #include "prefill.cuh"
 #include "stack_dev.cuh"
@@ -18,21 +20,20 @@
 
 namespace cq {
 
-constexpr int kTaBM = 128, kTaBN = 64;
-constexpr int kTaThreads = 320;                   // warp 0 TMA, warp 1 MMA, warps 2-9 softmax
-constexpr int kTaPTile = kTaBM * kTaBN * 2;       // 16 KB: [128 rows][64 keys]
-// Per head_dim HD (128 or 64): Q tile = HD / 64 blocks of [128 rows][128 bytes], K and V tiles = HD / 64 blocks of
-// [64 keys][128 bytes].  Q, K x 2, V x 2, P, barriers (the dynamic shared memory is declared 1024-byte aligned):
-// 113 KB for HD 128 and at most 102 registers, so two CTAs share an SM and one's softmax runs under the other's MMAs.
-// Twice 115,456 B and the 1 KB the system keeps per CTA fit an SM's 228 KB.
-__host__ __device__ constexpr int ta_q_tile(int hd) { return kTaBM * hd * 2; }
-__host__ __device__ constexpr int ta_k_tile(int hd) { return kTaBN * hd * 2; }
-__host__ __device__ constexpr int ta_smem(int hd) { return ta_q_tile(hd) + 4 * ta_k_tile(hd) + kTaPTile + 256 + 512; }   // + barriers, + the softmax warps' exchange words
-constexpr uint32_t kTaCols = 256;                 // TMEM columns: S x 2 (64 each), O (HD)
+constexpr int kTaBM = 128, kTaBN = 128, kTaQ = 2;      // queries of a tile, keys of a tile, query tiles of a CTA
+constexpr int kTaThreads = 320;
+// Per head_dim HD (128 or 64): a tile of Q, K or V = HD / 64 blocks of [128 rows][128 bytes].  Q x 2, K x 2, V x 2, barriers; the dynamic
+// shared memory is declared 1024-byte aligned.
+constexpr int kTaBlk = 128 * 128;
+__host__ __device__ constexpr int ta_tile(int hd) { return hd / 64 * kTaBlk; }
+__host__ __device__ constexpr int ta_smem(int hd) { return 6 * ta_tile(hd) + 256; }
+// TMEM columns: S (128; P in the first 64 of them) and O (HD, 128 at the most) of one query tile or two.  A launch of at most 128 queries takes
+// half of the memory, so that the next launch's first CTAs find some.
+__host__ __device__ constexpr uint32_t ta_cols(int T) { return T > kTaBM ? 512u : 256u; }
 
 struct PfAttnTcArgs {
     CUtensorMap tq;          // q as [T][ldq] fp16, box 64 x 128, swizzled
-    CUtensorMap tk, tv;      // caches as [n_kv][max_seq][hd] fp16, box 64 x 64 x 1, swizzled
+    CUtensorMap tk, tv;      // caches as [n_kv][rows][hd] fp16, box 64 x 128 x 1, swizzled
     __half* out;
     int T, pos0, n_heads, grp, ldq;
     float scale_log2;
@@ -40,186 +41,191 @@ struct PfAttnTcArgs {
 };
 
 __device__ __forceinline__ float ta_ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-__device__ __forceinline__ void ta_sts128(uint32_t addr, uint4 v) {
-    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
 
 template <int HD>
-__global__ void __launch_bounds__(kTaThreads, 2) prefill_attn_tc_kernel(const __grid_constant__ PfAttnTcArgs a) {
-    constexpr int kTaHD = HD, kTaQTile = ta_q_tile(HD), kTaQHalf = kTaBM * 128, kTaKTile = ta_k_tile(HD), kTaKHalf = kTaBN * 128, NBLK = HD / 64;
-    extern __shared__ __align__(1024) unsigned char ta_smem[];
-    const uint32_t base = smem_u32(ta_smem);
-    const uint32_t sQ = base, sK = base + kTaQTile, sV = sK + 2 * kTaKTile, sP = sV + 2 * kTaKTile;
-    const uint32_t bars = sP + kTaPTile;
-    const uint32_t b_q = bars, b_kvfull = bars + 8, b_kvfree = bars + 24, b_sfull = bars + 40, b_p = bars + 56, b_pv = bars + 64, tmem_slot = bars + 72;
+__global__ void __launch_bounds__(kTaThreads, 1) prefill_attn_tc_kernel(const __grid_constant__ PfAttnTcArgs a) {
+    constexpr int kTile = ta_tile(HD), NBLK = HD / 64;
+    extern __shared__ __align__(1024) unsigned char ta_smem_raw[];
+    const uint32_t base = smem_u32(ta_smem_raw);
+    const uint32_t sQ = base, sK = sQ + 2 * kTile, sV = sK + 2 * kTile, bars = sV + 2 * kTile;
+    const uint32_t b_q = bars, b_kfull = bars + 8, b_kfree = bars + 24, b_vfull = bars + 40, b_vfree = bars + 56, b_s = bars + 72, b_p = bars + 88, b_o = bars + 120, tmem_slot = bars + 136;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int head = blockIdx.y, kvh = head / a.grp;
-    const int q0 = (gridDim.x - 1 - blockIdx.x) * kTaBM;                  // the longest tiles first
-    const int kmax = a.pos0 + min(q0 + kTaBM, a.T);                      // keys [0, kmax) matter to this tile
-    const int nj = (kmax + kTaBN - 1) / kTaBN;
+    const int q0 = (gridDim.x - 1 - blockIdx.x) * (kTaQ * kTaBM);         // the longest tiles first
+    const int nq = q0 + kTaBM < a.T ? 2 : 1;                             // query tiles that have queries
+    auto key_end = [&](int i) { return a.pos0 + min(q0 + (i + 1) * kTaBM, a.T); };      // keys that query tile i sees at all
+    auto tiles = [&](int i) { return (key_end(i) + kTaBN - 1) / kTaBN; };               // its key tiles; the last query tile has the most
+    const int nj = tiles(nq - 1);
+    const uint32_t cols = ta_cols(a.T);
     bool failed = false;
 
     if (threadIdx.x == 0) {
         mbar_init(b_q, 1);
-        for (int s = 0; s < 2; ++s) { mbar_init(b_kvfull + 8 * s, 1); mbar_init(b_kvfree + 8 * s, 1); mbar_init(b_sfull + 8 * s, 1); }
-        mbar_init(b_p, 8); mbar_init(b_pv, 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(b_kfull + 8 * s, 1); mbar_init(b_kfree + 8 * s, 1); mbar_init(b_vfull + 8 * s, 1); mbar_init(b_vfree + 8 * s, 1);
+            mbar_init(b_s + 8 * s, 1); mbar_init(b_p + 16 * s, 4); mbar_init(b_p + 16 * s + 8, 4); mbar_init(b_o + 8 * s, 1);
+        }
         mbar_fence_init();
     }
-    if (warp == 1) { tmem_alloc(tmem_slot, kTaCols); tmem_relinquish(); }
+    if (warp == 9) { tmem_alloc(tmem_slot, cols); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = lds32(tmem_slot);
     pdl_launch_dependents();      // after the allocation: what the next launch takes early can not keep a CTA of this one waiting
-    const uint32_t tS = tmem, tO = tmem + 2u * kTaBN;
+    const uint32_t tS = tmem, tO = tmem + cols / 2;
 
-    if (warp == 0) {
+    if (warp == 8) {
         if (lane == 0) {
             pdl_wait();           // everything below follows from these loads
-            mbar_expect_tx(b_q, (uint32_t)kTaQTile);
-            for (int b = 0; b < NBLK; ++b) tma_load_2d(sQ + b * kTaQHalf, &a.tq, head * kTaHD + 64 * b, q0, b_q);
+            mbar_expect_tx(b_q, (uint32_t)(nq * kTile));
+            for (int i = 0; i < nq; ++i)
+                for (int b = 0; b < NBLK; ++b) tma_load_2d(sQ + i * kTile + b * kTaBlk, &a.tq, head * HD + 64 * b, q0 + i * kTaBM, b_q);
             for (int j = 0; j < nj; ++j) {
-                const int s = j & 1;
-                if (!mbar_wait(b_kvfree + 8 * s, (((uint32_t)j >> 1) & 1u) ^ 1u)) { failed = true; break; }
-                mbar_expect_tx(b_kvfull + 8 * s, 2u * kTaKTile);
-                for (int b = 0; b < NBLK; ++b) {
-                    tma_load_3d(sK + s * kTaKTile + b * kTaKHalf, &a.tk, 64 * b, j * kTaBN, kvh, b_kvfull + 8 * s);
-                    tma_load_3d(sV + s * kTaKTile + b * kTaKHalf, &a.tv, 64 * b, j * kTaBN, kvh, b_kvfull + 8 * s);
-                }
+                const int s = j & 1; const uint32_t free_par = (((uint32_t)j >> 1) & 1u) ^ 1u;
+                if (!mbar_wait(b_kfree + 8 * s, free_par)) { failed = true; break; }
+                mbar_expect_tx(b_kfull + 8 * s, (uint32_t)kTile);
+                for (int b = 0; b < NBLK; ++b) tma_load_3d(sK + s * kTile + b * kTaBlk, &a.tk, 64 * b, j * kTaBN, kvh, b_kfull + 8 * s);
+                if (!mbar_wait(b_vfree + 8 * s, free_par)) { failed = true; break; }
+                mbar_expect_tx(b_vfull + 8 * s, (uint32_t)kTile);
+                for (int b = 0; b < NBLK; ++b) tma_load_3d(sV + s * kTile + b * kTaBlk, &a.tv, 64 * b, j * kTaBN, kvh, b_vfull + 8 * s);
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == 9) {
         if (lane == 0) {
-            constexpr uint32_t idS = umma_idesc_f16(kTaBM, kTaBN, 0), idPV = umma_idesc_f16(kTaBM, kTaHD, 1);
-            auto issue_s = [&](int j) -> bool {
+            constexpr uint32_t idS = umma_idesc_f16(kTaBM, kTaBN, 0), idPV = umma_idesc_f16(kTaBM, HD, 1);
+            // S of query tile i and key tile j; the last query tile's reads the K slot last
+            auto issue_s = [&](int i, int j) {
                 const int s = j & 1;
-                if (!mbar_wait(b_kvfull + 8 * s, ((uint32_t)j >> 1) & 1u)) return false;
-                tc_fence_after();
 #pragma unroll
-                for (int ks = 0; ks < kTaHD / 16; ++ks) {
-                    umma_f16(tS + (uint32_t)(s * kTaBN), umma_desc_sw128(sQ + (uint32_t)((ks >> 2) * kTaQHalf + (ks & 3) * 32), 16, 1024),
-                             umma_desc_sw128(sK + s * kTaKTile + (uint32_t)((ks >> 2) * kTaKHalf + (ks & 3) * 32), 16, 1024), idS, (uint32_t)(ks != 0));
+                for (int ks = 0; ks < HD / 16; ++ks) {
+                    const uint32_t off = (uint32_t)((ks >> 2) * kTaBlk + (ks & 3) * 32);
+                    umma_f16(tS + (uint32_t)(i * kTaBN), umma_desc_sw128(sQ + i * kTile + off, 16, 1024), umma_desc_sw128(sK + s * kTile + off, 16, 1024), idS, (uint32_t)(ks != 0));
                 }
-                umma_commit(b_sfull + 8 * s);
-                return true;
+                umma_commit(b_s + 8 * i);
+                if (i == nq - 1) umma_commit(b_kfree + 8 * s);
             };
-            if (!mbar_wait(b_q, 0u)) failed = true;
-            if (!failed && !issue_s(0)) failed = true;
+            if (!mbar_wait(b_q, 0u) || !mbar_wait(b_kfull, 0u)) failed = true;
+            tc_fence_after();
+            if (!failed) for (int i = 0; i < nq; ++i) issue_s(i, 0);
             for (int j = 0; j < nj && !failed; ++j) {
                 const int s = j & 1;
-                if (j + 1 < nj && !issue_s(j + 1)) { failed = true; break; }
-                if (!mbar_wait(b_p, (uint32_t)j & 1u)) { failed = true; break; }
-                tc_fence_after();
+                if (!mbar_wait(b_vfull + 8 * s, ((uint32_t)j >> 1) & 1u)) { failed = true; break; }
+                if (j + 1 < nj && !mbar_wait(b_kfull + 8 * (s ^ 1), ((uint32_t)(j + 1) >> 1) & 1u)) { failed = true; break; }
+                for (int i = 0; i < nq && !failed; ++i) {
+                    const int mine = tiles(i);
+                    if (j >= mine) continue;
+                    const int steps = min(kTaBN / 32, (key_end(i) - j * kTaBN + 31) / 32) * 2;
+                    for (int half = 0; half < 2; ++half) {        // P arrives in halves of 64 keys
+                        if (!mbar_wait(b_p + 16 * i + 8 * half, (uint32_t)j & 1u)) { failed = true; break; }
+                        tc_fence_after();
 #pragma unroll
-                for (int ks = 0; ks < kTaBN / 16; ++ks)       // sixteen keys a step: V rows 16 ks .., P columns 16 ks ..
-                    umma_f16(tO, umma_desc_sw128(sP + (uint32_t)(ks * 32), 16, 1024),
-                             umma_desc_sw128(sV + s * kTaKTile + ks * 2048, kTaKHalf, 1024), idPV, (uint32_t)((j | ks) != 0));
-                umma_commit(b_pv);
-                umma_commit(b_kvfree + 8 * s);
+                        for (int k4 = 0; k4 < 4; ++k4) {          // sixteen keys a step: V rows 16 ks .., P columns 16 ks .. (two to a 32-bit column)
+                            const int ks = half * 4 + k4;
+                            if (ks < steps) umma_f16_ta(tO + (uint32_t)(i * HD), tS + (uint32_t)(i * kTaBN + ks * 8), umma_desc_sw128(sV + s * kTile + ks * 2048, kTaBlk, 1024), idPV, (uint32_t)((j | ks) != 0));
+                        }
+                    }
+                    if (failed) break;
+                    if (i == nq - 1) umma_commit(b_vfree + 8 * s);
+                    if (j + 1 < mine) issue_s(i, j + 1);
+                    else umma_commit(b_o + 8 * i);
+                }
             }
         }
-    } else {
-        // Eight softmax warps: two per TMEM lane quarter (a warp reaches the 32 lanes its number mod 4 names), each with
-        // 32 of a tile's 64 keys and half of the output columns of the same 32 query rows.  The two threads of a row
-        // agree on the row's scaling exponent through 512 bytes of shared memory and two named barriers per tile - so
-        // nothing below leaves the tile loop early: after a wait has run out the warp keeps going without waiting.
-        const int q = warp & 3, hsel = (warp - 2) >> 2;
-        const int r = q * 32 + lane;                                      // query row of the tile = TMEM lane
-        const int qpos = a.pos0 + q0 + r;
-        const uint32_t lane_off = (uint32_t)(q * 32) << 16;
-        __half* mxbuf = reinterpret_cast<__half*>(ta_smem + (bars - base) + 256);      // [2 halves][128 rows]
-        constexpr int OC = HD / 2;                                        // output columns of this thread
+    } else if ((warp >> 2) < nq) {
+        const int i = warp >> 2, r = (warp & 3) * 32 + lane;              // query tile, row of it = TMEM lane
+        const int qpos = a.pos0 + q0 + i * kTaBM + r, mine = tiles(i);
+        const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16, s_at = tS + (uint32_t)(i * kTaBN) + lane_off, o_at = tO + (uint32_t)(i * HD) + lane_off;
         // m is the exponent the row's probabilities are scaled by, not always its running maximum: it moves only when
         // a tile's maximum exceeds it by more than 2^8 (probabilities then stay below 256, well inside fp16, and the
         // row sum is fp32), so that most tiles need no rescale of O in TMEM.
         float m = -INFINITY, l = 0.f;
-        for (int j = 0; j < nj; ++j) {
-            const int s = j & 1;
-            if (!failed && !mbar_wait(b_sfull + 8 * s, ((uint32_t)j >> 1) & 1u)) failed = true;
+        const f32x2 scale2 = pack2(a.scale_log2, a.scale_log2);
+        for (int j = 0; j < mine; ++j) {
+            if (!failed && !mbar_wait(b_s + 8 * i, (uint32_t)j & 1u)) failed = true;
             tc_fence_after();
-            const bool diag = j * kTaBN + kTaBN - 1 > a.pos0 + q0;        // some key of this tile may lie past some query (uniform over the CTA)
-            float x[32];
-            tmem_ld32(tS + (uint32_t)(s * kTaBN + hsel * 32) + lane_off, x);
-            float mxl = -INFINITY;
+            const int key0 = j * kTaBN, nc = min(4, (key_end(i) - key0 + 31) / 32);       // 32-key pieces that some query sees (uniform over the tile); P V leaves the others out
+            uint32_t x[4][32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                x[i] *= a.scale_log2;
-                if (diag && j * kTaBN + hsel * 32 + i > qpos) x[i] = -INFINITY;
-                mxl = fmaxf(mxl, x[i]);
-            }
-            const __half hmx = __float2half_ru(mxl);                      // rounded up: both threads of the row then hold the same two numbers
-            mxbuf[hsel * 128 + r] = hmx;
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            const float mx = fmaxf(__half2float(hmx), __half2float(mxbuf[(hsel ^ 1) * 128 + r]));
-            asm volatile("bar.sync 1, 256;" ::: "memory");                // everybody has read before the next tile's maxima are written
-            float alpha = 1.f;
-            const bool mine = mx > m + 8.0f;                              // also true on the first tile (m = -inf; key 0 is visible to every query)
-            const bool moved = __any_sync(0xffffffffu, mine);             // warp-uniform (the TMEM accesses below are warp-wide); the row's other warp decides alike
-            if (mine) { alpha = m == -INFINITY ? 0.f : ta_ex2(m - mx); m = mx; }
-            float rs = 0.f;
-            uint32_t pk[16];
+            for (int c = 0; c < 4; ++c) if (c < nc) tmem_ld32_issue(s_at + (uint32_t)(c * 32), x[c]);
+            tmem_wait_ld();
+            float mx4[4];
 #pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-                const float e0 = ta_ex2(x[i] - m), e1 = ta_ex2(x[i + 1] - m);
-                rs += e0 + e1;
-                pk[i >> 1] = pack_h2(e0, e1);
+            for (int c = 0; c < 4; ++c) {
+                mx4[c] = -INFINITY;
+                if (c >= nc) continue;
+                const int key = key0 + c * 32;
+                if (key + 31 > a.pos0 + q0 + i * kTaBM) {                 // some key of this piece may lie past some query (uniform over the tile)
+#pragma unroll
+                    for (int k = 0; k < 32; ++k) if (key + k > qpos) x[c][k] = 0xff800000u;      // -infinity
+                }
+#pragma unroll
+                for (int k = 0; k < 32; ++k) mx4[c] = fmaxf(mx4[c], __uint_as_float(x[c][k]));
             }
-            if (j > 0) {
-                if (!failed && !mbar_wait(b_pv, (uint32_t)(j - 1) & 1u)) failed = true;   // P V of the previous tile is complete: O and the P tile are ours
-                tc_fence_after();
-                if (moved) {
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * a.scale_log2;
+            const bool move = mx > m + 8.0f;                              // also true on the first tile (m = -inf; key 0 is visible to every query)
+            if (__any_sync(0xffffffffu, move)) {                          // warp-uniform: the TMEM accesses below are warp-wide
+                float alpha = 1.f;
+                if (move) { alpha = m == -INFINITY ? 0.f : ta_ex2(m - mx); m = mx; l *= alpha; }
+                if (j > 0) {
 #pragma unroll 1
-                    for (int c = 0; c < OC / 32; ++c) {
+                    for (int c = 0; c < HD / 32; ++c) {
                         float v[32];
-                        tmem_ld32(tO + lane_off + (uint32_t)(hsel * OC + c * 32), v);
+                        tmem_ld32(o_at + (uint32_t)(c * 32), v);
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) v[i] *= alpha;
-                        tmem_st32(tO + lane_off + (uint32_t)(hsel * OC + c * 32), v);
+                        for (int k = 0; k < 32; ++k) v[k] *= alpha;
+                        tmem_st32(o_at + (uint32_t)(c * 32), v);
                     }
+                }
+            }
+            const f32x2 m2 = pack2(-m, -m);
+            f32x2 sum[2] = {0ull, 0ull};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                if (c < nc) {
+                    uint32_t pk[16];
+#pragma unroll
+                    for (int k = 0; k < 32; k += 2) {
+                        float e0, e1;
+                        unpack2(fma2(pack2(__uint_as_float(x[c][k]), __uint_as_float(x[c][k + 1])), scale2, m2), e0, e1);
+                        e0 = ta_ex2(e0); e1 = ta_ex2(e1);
+                        sum[(k >> 1) & 1] = add2(sum[(k >> 1) & 1], pack2(e0, e1));
+                        pk[k >> 1] = pack_h2(e0, e1);
+                    }
+                    tmem_st16(s_at + (uint32_t)(c * 16), pk);
+                }
+                if (c & 1) {
                     tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(b_p + 16 * i + 8 * (c >> 1));
                 }
             }
-            const uint32_t prow = sP + (uint32_t)(r * 128);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                ta_sts128(prow + ((uint32_t)((hsel * 4 + i) ^ (r & 7)) << 4), make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]));
-            l = l * alpha + rs;
-            fence_async_smem();                                           // the tensor core reads P through the async proxy
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(b_p);
+            l += sum2(add2(sum[0], sum[1]));
         }
-        // the row's sum: the second half hands its part to the first, which hands back the total
-        float* lbuf = reinterpret_cast<float*>(mxbuf);                    // 128 floats
-        if (hsel == 1) lbuf[r] = l;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (hsel == 0) { l += lbuf[r]; lbuf[r] = l; }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (hsel == 1) l = lbuf[r];
-        if (!failed && !mbar_wait(b_pv, (uint32_t)(nj - 1) & 1u)) failed = true;
+        if (!failed && !mbar_wait(b_o + 8 * i, 0u)) failed = true;
         tc_fence_after();
-        {
-            const float inv = 1.0f / l;
-            const int t = q0 + r;
+        const float inv = 1.0f / l;
+        const int t = q0 + i * kTaBM + r;
 #pragma unroll 1
-            for (int c = 0; c < OC / 32; ++c) {
-                float v[32];
-                tmem_ld32(tO + lane_off + (uint32_t)(hsel * OC + c * 32), v);
-                if (t < a.T && !failed) {
-                    __half* dst = a.out + (size_t)t * a.ldq + head * kTaHD + hsel * OC + c * 32;
+        for (int c = 0; c < HD / 32; ++c) {
+            float v[32];
+            tmem_ld32(o_at + (uint32_t)(c * 32), v);
+            if (t < a.T && !failed) {
+                __half* dst = a.out + (size_t)t * a.ldq + head * HD + c * 32;
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8)
-                        *reinterpret_cast<uint4*>(dst + i) = make_uint4(pack_h2(v[i] * inv, v[i + 1] * inv), pack_h2(v[i + 2] * inv, v[i + 3] * inv),
-                                                                        pack_h2(v[i + 4] * inv, v[i + 5] * inv), pack_h2(v[i + 6] * inv, v[i + 7] * inv));
-                }
-                __syncwarp();
+                for (int k = 0; k < 32; k += 8)
+                    *reinterpret_cast<uint4*>(dst + k) = make_uint4(pack_h2(v[k] * inv, v[k + 1] * inv), pack_h2(v[k + 2] * inv, v[k + 3] * inv),
+                                                                    pack_h2(v[k + 4] * inv, v[k + 5] * inv), pack_h2(v[k + 6] * inv, v[k + 7] * inv));
             }
+            __syncwarp();
         }
     }
     if (failed && a.err) atomicExch(a.err, 12u);
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, kTaCols);
+    if (warp == 9) tmem_dealloc(tmem, cols);
 }
 
 typedef CUresult (*TaEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -262,14 +268,14 @@ int launch_prefill_attn_tc(int head_dim, const PfAttnArgs& a, int n_kv, unsigned
     const __half* caches[2] = {a.kc, a.vc};
     CUtensorMap* maps[2] = {&k.tk, &k.tv};
     for (int i = 0; i < 2; ++i) {
-        const cuuint64_t dims[3] = {(cuuint64_t)kTaHD, (cuuint64_t)a.max_seq, (cuuint64_t)n_kv};
+        const cuuint64_t dims[3] = {(cuuint64_t)kTaHD, (cuuint64_t)(a.pos0 + a.T), (cuuint64_t)n_kv};      // rows past the last query's arrive as zeros, whatever the cache holds there
         const cuuint64_t strides[2] = {(cuuint64_t)kTaHD * 2, (cuuint64_t)a.max_seq * kTaHD * 2};
         const cuuint32_t box[3] = {64, kTaBN, 1};
         if (fn(maps[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half*>(caches[i]), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return (int)cudaErrorInvalidValue;
     }
     k.out = a.out; k.T = a.T; k.pos0 = a.pos0; k.n_heads = a.n_heads; k.grp = a.grp; k.ldq = a.ldq; k.scale_log2 = a.scale_log2; k.err = err;
-    const dim3 grid((a.T + kTaBM - 1) / kTaBM, a.n_heads);
+    const dim3 grid((a.T + kTaQ * kTaBM - 1) / (kTaQ * kTaBM), a.n_heads);
     return head_dim == 128 ? ta_go<128>(k, grid, cfg) : ta_go<64>(k, grid, cfg);
 }
 

@@ -328,3 +328,28 @@ def test_prefill_attention_kernels(built, impl, hd, T, pos0, nh, nkv):
     got = out.numpy(np.float16).reshape(T, nh * hd)
     assert np.isfinite(got.astype(np.float32)).all()
     assert close(got, want), report(got, want)
+
+
+# edges of the 128-query and 128-key tiles, of the two query tiles of a CTA and of the 32-key pieces of a last tile
+@pytest.mark.parametrize("hd", [128, 64])
+@pytest.mark.parametrize("T,pos0,nh,nkv", [(2, 31, 2, 1), (32, 0, 2, 1), (33, 0, 2, 1), (97, 30, 2, 2), (127, 1, 2, 1), (128, 0, 2, 1), (129, 0, 3, 1), (255, 0, 2, 1), (256, 0, 2, 1), (257, 127, 2, 1),
+                                           (384, 128, 2, 1), (385, 1000, 2, 1), (640, 63, 2, 1)])
+def test_prefill_attention_at_tile_edges(built, hd, T, pos0, nh, nkv):
+    test_prefill_attention_kernels(built, 0, hd, T, pos0, nh, nkv)
+
+
+@pytest.mark.parametrize("hd", [128, 64])
+def test_prefill_attention_moves_its_exponent(built, hd):
+    """Scores that grow from key tile to key tile by far more than 2^8, so that every tile rescales what has been summed."""
+    rng = np.random.default_rng(hd)
+    T, nh, nkv, max_seq = 300, 2, 1, 640
+    q = np.abs(rng.standard_normal((T, nh * hd))).astype(np.float16)
+    Kc = rng.standard_normal((nkv, max_seq, hd)).astype(np.float16)
+    Kc += (np.arange(max_seq) // 100 * 0.5).astype(np.float16)[None, :, None]
+    Vc = rng.standard_normal((nkv, max_seq, hd)).astype(np.float16)
+    out = DevBuf(T * nh * hd * 2)
+    K.prefill_attention(0, dev(q), dev(Kc), dev(Vc), out, T, 330, nh, nkv, hd, max_seq)
+    sync()
+    want = attn_oracle(q, Kc, Vc, 330, nh, nkv, hd)
+    got = out.numpy(np.float16).reshape(T, nh * hd)
+    assert close(got, want), report(got, want)
