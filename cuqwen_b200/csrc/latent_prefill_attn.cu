@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(kLpThreads, 2) latent_prefill_attn_kernel(cons
     const int nj = (p_last + 1 - k_first + kLpBN - 1) / kLpBN;
     bool failed = false;
 
+    if (threadIdx.x == 64) { prefetch_map(&a.tqn); prefetch_map(&a.tkn); prefetch_map(&a.tv); if (a.nbr) { prefetch_map(&a.tqr); prefetch_map(&a.tkr); } }
     if (threadIdx.x == 0) {
         mbar_init(b_q, 1);
         for (int s = 0; s < 2; ++s) { mbar_init(b_kfull + 8 * s, 1); mbar_init(b_kfree + 8 * s, 1); mbar_init(b_vfull + 8 * s, 1); mbar_init(b_vfree + 8 * s, 1); mbar_init(b_sfull + 8 * s, 1); }

@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) prefill_attn_tc_kernel(const __
     const uint32_t cols = ta_cols(a.T);
     bool failed = false;
 
+    if (threadIdx.x == 256) { prefetch_map(&a.tq); prefetch_map(&a.tk); prefetch_map(&a.tv); }
     if (threadIdx.x == 0) {
         mbar_init(b_q, 1);
         for (int s = 0; s < 2; ++s) {

@@ -180,7 +180,9 @@ __global__ void __launch_bounds__(kPfThreads, NT == 64 ? 2 : 1) prefill_gemm_ker
     constexpr int kRawKb = Q == Q_I4 ? 32 : 64;               // raw bytes of one row in one K block
     bool failed = false;
 
+    if (threadIdx.x == 32) { prefetch_map(&a.tx); if (Q == Q_BF16 && a.K2 > 0) { prefetch_map(&a.tx2); prefetch_map(&a.tw2); } }
     if (threadIdx.x == 0) {
+        prefetch_map(&a.tw[CG == 2 && swiglu ? rank : seg]);
         for (int s = 0; s < NA; ++s) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_afree + 8 * s, 1); }
         for (int s = 0; s < NB; ++s) { mbar_init(bar_conv + 8 * s, CG == 1 ? kPfConvWarps : kRaw ? 2 * kPfConvWarps : 1); mbar_init(bar_bfree + 8 * s, 1); }
         mbar_init(bar_done, 1);
