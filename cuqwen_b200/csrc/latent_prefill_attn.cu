@@ -1,6 +1,6 @@
 // Windowed attention of a portion's queries over per-head keys and values with a shared rotated key part, a sink and an
-// output gate, in bfloat16 on the tcgen05 tensor cores: prefill_attn_tc.cu's scheme with query / key rows in two parts
-// (unrotated, per head; rotated, one for all heads), any lengths, and the first visible key as the first tile's start.
+// output gate, in bfloat16 on the tcgen05 tensor cores: query / key rows in two parts (unrotated, per head; rotated, one for all
+// heads), any lengths, and the first visible key as the first tile's start.
 //
 // One CTA = 128 queries of one head.  Per tile of 64 keys:
 //   warp 0      TMA: the two key parts and the values in 64-column swizzled boxes (columns past a part's end arrive as
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kLpThreads, 2) latent_prefill_attn_kernel(cons
             }
         }
     } else {
-        // As in prefill_attn_tc.cu: warp w reaches the TMEM lanes 32 (w mod 4) ..; the two threads of a row agree on m through
+        // Warp w reaches the TMEM lanes 32 (w mod 4) ..; the two threads of a row agree on m through
         // shared memory; nothing leaves the loop early, after a failed wait a warp goes on without waiting.
         const int q = warp & 3, hsel = (warp - 2) >> 2, r = q * 32 + lane, qpos = p_first + r;
         const uint32_t lane_off = (uint32_t)(q * 32) << 16;

@@ -1,6 +1,6 @@
 // Causal attention for a tile of prompt tokens on the tcgen05 tensor cores (head_dim 64 or 128): the batched counterpart of
 // the reference's decode attention (src/kernels.cu:105-288), which the reference applies once per prompt token
-// (src/main.cu:86-92).  prefill_attn.cu holds an mma.sync kernel for comparison.
+// (src/main.cu:86-92).  prefill_attn.cu holds an mma.sync kernel, used for few queries near the beginning.
 //
 // One CTA = two tiles of 128 queries of one head, one CTA to an SM.  Per tile of 128 keys:
 //   warp 8      TMA: K and V tiles of the head's KV group (64-column boxes, hardware-swizzled), two slots each
@@ -11,7 +11,8 @@
 //               and O is rescaled in TMEM by 2^(m_old - m_new) (rare after the first tiles)
 // While one tile's softmax runs, the tensor core works for the other.  A row belongs to one thread and P stays in tensor memory, so a tile costs
 // no barrier among the softmax warps and no pass through shared memory; what bounds it is the chain of a tile - scores, exponentials (1024
-// cycles of an SM partition's unit), P V, next scores - of which the two query tiles hide half.
+// cycles of an SM partition's unit), P V, next scores - of which the two query tiles hide half.  Against two threads to a row, P in shared
+// memory, 64-key tiles and two CTAs to an SM: 40 heads x 8190 queries 782 us for 999 (0.88 PFLOP/s), 16 heads x 3000 queries at 1000 115 for 140.
 // The tensor core finishes its MMAs in the order of issue: when S of a key tile is there, so is P V of the one before, and O may be rescaled.
 // Every mbarrier wait is bounded; a wait that runs out sets *err and the CTA drains.
 #include "prefill.cuh"
