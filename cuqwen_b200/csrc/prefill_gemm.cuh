@@ -30,7 +30,6 @@
 namespace cq {
 
 constexpr int kPfM = 128;            // tokens per tile
-constexpr int kPfN = 256;            // weight rows per tile at the most (two matrices of half as many rows each in the SwiGLU mode)
 constexpr int kPfKB = 64;            // K per pipeline stage: 128 bytes of fp16, one swizzle row
 constexpr int kPfConvWarps = 8;      // 8: a weight row of a K block per thread; 16: half a row (measured: no faster, the kernel is bound elsewhere)
 constexpr int kPfThreads = (2 + kPfConvWarps) * 32;
