@@ -103,7 +103,7 @@ static int dev_ctx(int device, DevCtx** out) {
         CK(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device));
         CK(cudaEventCreate(&d.ev0)); CK(cudaEventCreate(&d.ev1));
         CK(cudaEventCreateWithFlags(&d.ev_join, cudaEventDisableTiming));
-        CK(cudaMalloc((void**)&d.err, 4)); CK(cudaMemset(d.err, 0, 4)); CK(cudaMallocHost((void**)&d.h_err, 4));
+        CK(cudaMalloc((void**)&d.err, 4)); CK(cudaMemsetAsync(d.err, 0, 4, d.stream)); CK(cudaMallocHost((void**)&d.h_err, 4));
         d.init = true;
     }
     *out = &d;
@@ -410,7 +410,7 @@ extern "C" int cuqwen_load(cuqwen_engine* e, const char* path) {
     if (e->p.flags & CUQWEN_FLAG_STEP_TRACE) {      // eight timeline words per launch, zeroed by the reader between steps
         e->step_trace_bytes = (size_t)(1 + 8 * e->p.n_layers + 8) * kTraceWords * 8;
         CK(cudaMalloc((void**)&e->step_trace, e->step_trace_bytes));
-        CK(cudaMemset(e->step_trace, 0, e->step_trace_bytes));
+        CK(cudaMemsetAsync(e->step_trace, 0, e->step_trace_bytes, e->stream));
     }
     e->loaded = true;
     return CUQWEN_OK;
@@ -728,7 +728,7 @@ static int check_tokens(const cuqwen_engine* e, const int* tokens, int n_tokens,
 static int stack_portion(cuqwen_engine* e, const int* tokens, int n_tokens, int pos0, const int* want, int n_want, float* logits) {
     const int C = stack_chunk();
     CK(cudaSetDevice(e->p.device));
-    if (int r = stack_workspace(e->stack, std::min(n_tokens, C))) return r;
+    if (int r = stack_workspace(e, std::min(n_tokens, C))) return r;
     if (int r = stack_begin(e->stack, pos0)) return r;
     t_err = reinterpret_cast<unsigned*>(&e->ctl->pad[0]);
     if (!e->pf_tok) CK(cudaMalloc((void**)&e->pf_tok, (size_t)C * 4));
@@ -1120,7 +1120,7 @@ extern "C" int cuqwen_dev_sync(int device) {
     DEV(device); (void)cfg;
     CK(cudaMemcpyAsync(dc->h_err, dc->err, 4, cudaMemcpyDeviceToHost, dc->stream));
     CK(cudaStreamSynchronize(dc->stream)); CK(cudaGetLastError());
-    if (*dc->h_err) { unsigned c = *dc->h_err; CK(cudaMemset(dc->err, 0, 4)); return fail(CUQWEN_ERR_TIMEOUT, "a bounded device-side wait expired (code %u)", c); }
+    if (*dc->h_err) { unsigned c = *dc->h_err; CK(cudaMemsetAsync(dc->err, 0, 4, dc->stream)); return fail(CUQWEN_ERR_TIMEOUT, "a bounded device-side wait expired (code %u)", c); }
     return CUQWEN_OK;
 }
 // Orders the library's per-device stream against a caller's stream (0 = the legacy default stream):

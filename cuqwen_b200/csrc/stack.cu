@@ -31,7 +31,8 @@ int stack_begin(Stack* s, int pos0) {
 }
 void stack_end(Stack* s, int pos) { s->next_pos = pos; }
 
-static int alloc_ws(Stack* s, Stack::Ws* w, int rows, bool decode) {
+// The zeros (padding is read) come on the stream that the work follows on: it does not wait for the default stream.
+static int alloc_ws(cuqwen_engine* e, Stack* s, Stack::Ws* w, int rows, bool decode) {
     Arena2 dry, real;
     for (int pass = 0; pass < 2; ++pass) {
         Arena2& a = pass ? real : dry;
@@ -63,7 +64,7 @@ static int alloc_ws(Stack* s, Stack::Ws* w, int rows, bool decode) {
         }
         if (!pass) {
             SK(cudaMalloc((void**)&w->arena, dry.used + 256));
-            SK(cudaMemset(w->arena, 0, dry.used + 256));
+            SK(cudaMemsetAsync(w->arena, 0, dry.used + 256, e->stream));
             real.base = w->arena; real.dry = false;
         }
     }
@@ -140,7 +141,7 @@ int stack_create(cuqwen_engine* e, const StackSpec& spec, int act, int max_seq_l
         s->rot_tables.push_back(t);
         SK(launch_rot_table(t, max_seq_len, r.dims, r.base, LaunchCfg{e->stream, e->sms, false}));
     }
-    if (int r = alloc_ws(s, &s->dec, 1, true)) return r;
+    if (int r = alloc_ws(e, s, &s->dec, 1, true)) return r;
     SK(cudaMalloc((void**)&s->logits, (size_t)s->vocab_p * 4)); SK(cudaMemset(s->logits, 0, (size_t)s->vocab_p * 4));
     e->p.model_id = CUQWEN_MODEL_CUSTOM; e->p.vocab_size = spec.vocab; e->p.dim = spec.width; e->p.n_layers = (int)spec.layers.size();
     const LayerSpec& first = spec.layers[0];
@@ -548,7 +549,8 @@ int stack_record_step(cuqwen_engine* e, const LaunchCfg& cfg, const std::functio
 }
 
 // Workspace of a portion: rows for the longest so far, at least twice as many when it has to grow.  No portion is in flight here.
-int stack_workspace(Stack* s, int need) {
+int stack_workspace(cuqwen_engine* e, int need) {
+    Stack* s = e->stack;
     if (!s->logits_rows) {
         if (!s->xn_rows) SK(cudaMalloc((void**)&s->xn_rows, (size_t)kLogitRows * s->wp * s->esz));
         if (!s->want_rows) SK(cudaMalloc((void**)&s->want_rows, (size_t)kChunk * 4));
@@ -558,7 +560,7 @@ int stack_workspace(Stack* s, int need) {
     const int most = kChunk < s->max_seq ? kChunk : s->max_seq, rows = (need + 255) / 256 * 256, twice = 2 * s->pf.rows, want = rows > twice ? rows : twice;
     if (s->pf.arena) SK(cudaFree(s->pf.arena));
     s->pf = Stack::Ws{};
-    return alloc_ws(s, &s->pf, want < most ? want : most, false);
+    return alloc_ws(e, s, &s->pf, want < most ? want : most, false);
 }
 
 int stack_run_chunk(cuqwen_engine* e, int T, int pos0, const int* want, int n_want, float* logits_host) {

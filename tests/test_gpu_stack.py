@@ -337,6 +337,21 @@ def test_portions_beyond_4096_tokens(models):
 
 
 @pytest.mark.parametrize("act", ACTS)
+def test_a_sequence_goes_on_through_a_workspace_that_grows(models, act):
+    """300 tokens, 700 more and 4100 more in a chat's order: each portion outgrows the workspace of the one before, and the last crosses the
+    border at which a portion is cut."""
+    d, cfg, wf, _, _ = models("small")
+    n = 5100
+    toks = np.random.default_rng(6).integers(0, cfg["vocab"], n)
+    eng = E.Engine.open(d, act=act, max_seq_len=n)
+    for at, end in ((0, 300), (300, 1000), (1000, n)):
+        places = [p for p in (40, 255, 299, 300, 301, 308, 364, 998, 999, 1000, 1001, 1008, 1064, 4095, 4096, 5094, 5095, 5096, 5097, n - 1) if at <= p < end]
+        got = eng.extend(toks[at:end], at, [p - at for p in places])
+        check(got, np.concatenate([L.forward(cfg, wf, toks[p - 40:p + 1])[-1:] for p in places]), act, 1.5)
+    eng.close()
+
+
+@pytest.mark.parametrize("act", ACTS)
 def test_generation_through_step_decode_and_command_line(models, act):
     d, cfg, wf, _, _ = models("small")
     prompt, n = [5, 17, 3, 88, 41, 2, 60], 24

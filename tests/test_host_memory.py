@@ -1,0 +1,75 @@
+"""What portions do with device memory, on the CPU: the library runs over tests/cudart_stub.cpp (no kernels; device memory is host
+memory under a limit), each case in a process of its own."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+from cuqwen_b200 import binfmt, build
+from cuqwen_b200 import stackfmt as F
+import mixer_util
+import stack_util
+
+ROOT = Path(__file__).resolve().parent.parent
+TABLE = dict(vocab=512, dim=256, inter=512, layers=2, heads=2, kv=1, hd=128, tied=True)
+PRELUDE = """
+import ctypes, os, sys
+import numpy as np
+from cuqwen_b200 import CuQwenError
+from cuqwen_b200 import engine as E
+stub = ctypes.CDLL(os.environ["LD_PRELOAD"])
+stub.stub_limit.argtypes = [ctypes.c_size_t]
+stub.stub_used.restype = stub.stub_peak.restype = ctypes.c_size_t
+stub.stub_unordered.restype = ctypes.c_long
+stub.stub_copies.restype = ctypes.c_char_p
+copies = lambda: [int(n) for n in stub.stub_copies().split()]
+toks = np.arange(20000, dtype=np.int32) % 50
+"""
+
+
+@pytest.fixture(scope="module")
+def run(built, tmp_path_factory):
+    """run(code, *args): a fresh interpreter with the stub in place of the CUDA runtime; its standard output."""
+    lib = tmp_path_factory.mktemp("stub") / "libcudart_stub.so"
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", f"-I{build.cuda_home() / 'include'}", str(ROOT / "tests" / "cudart_stub.cpp"), "-o", str(lib)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+    def go(code, *args):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + code, *map(str, args)], capture_output=True, text=True, timeout=300, cwd=ROOT,
+                           env={**os.environ, "LD_PRELOAD": str(lib), "PYTHONPATH": str(ROOT)})
+        assert r.returncode == 0, r.stdout + r.stderr
+        return r.stdout
+    return go
+
+
+@pytest.fixture(scope="module")
+def directories(tmp_path_factory):
+    out = {}
+    for name, cfg, w in (("falivik", stack_util.small(), None), ("gipotar", mixer_util.small(), mixer_util.weights("small", 11)[1])):
+        out[name] = F.write_model_dir(tmp_path_factory.mktemp(name), cfg, w or stack_util.weights(cfg, 11)[0])
+    return out
+
+
+@pytest.fixture(scope="module")
+def table_file(tmp_path_factory):
+    path = tmp_path_factory.mktemp("table") / "m.bin"
+    binfmt.write_model(path, TABLE, 2, binfmt.random_tensors(TABLE, 3))
+    return path
+
+
+@pytest.mark.parametrize("act", ["float32", "bfloat16"])
+@pytest.mark.parametrize("design", ["falivik", "gipotar"])
+def test_nothing_runs_beside_a_fill_of_its_workspace(run, directories, design, act):
+    """The engine's stream does not wait for the default stream: a workspace that grows is cleared on the stream that uses it."""
+    run("""
+eng = E.Engine.open(sys.argv[1], act=sys.argv[2], max_seq_len=5200)
+stub.stub_unordered()
+at = 0
+for n in (300, 700, 4100):
+    eng.extend(toks[:n], at, [n - 1])
+    assert stub.stub_unordered() == 0, n
+    at += n
+""", directories[design], act)
