@@ -23,6 +23,7 @@
 #include "errors.h"
 #include "gemv.cuh"
 #include "launch.h"
+#include "portion.h"
 #include "prefill.cuh"
 #include "prefill_gemm.cuh"
 #include "gemv_seg.cuh"
@@ -694,17 +695,25 @@ extern "C" int cuqwen_step(cuqwen_engine* e, int token, int pos, const int* hist
 constexpr int kPrefillChunk = 8192;
 #define PK(call) do { int r_ = (call); if (r_) return fail(r_ == (int)cudaErrorInvalidValue ? CUQWEN_ERR_ARG : CUQWEN_ERR_CUDA, "%s: %s", #call, cudaGetErrorString((cudaError_t)r_)); } while (0)
 
-// The workspace holds as many tokens as the longest portion so far, rounded up; a portion beyond it gets a new one of at least twice the size.
-static int prefill_workspace(cuqwen_engine* e, int need) {
-    if (need <= e->pf_rows) return CUQWEN_OK;
+// The workspace holds as many tokens as the longest portion so far, rounded up (portion.h); *rows: how many go through the layers together.
+static int prefill_workspace(cuqwen_engine* e, int need, int* rows) {
     const cuqwen_params& p = e->p;
-    const size_t C = (size_t)std::min(kPrefillChunk, std::max((need + 255) / 256 * 256, 2 * e->pf_rows)), qd = (size_t)e->q_dim_l, kd = (size_t)e->kv_dim_l;
-    struct { void** at; size_t bytes; } const bufs[] = {{(void**)&e->pf_x, C * p.dim * 2}, {(void**)&e->pf_xn, C * p.dim * 2}, {(void**)&e->pf_qkv, C * (qd + 2 * kd) * 4}, {(void**)&e->pf_q, C * qd * 2},
-                                                        {(void**)&e->pf_att, C * qd * 2}, {(void**)&e->pf_g, C * e->inter_l * 2}, {(void**)&e->pf_tok, C * 4}};
-    e->pf_rows = 0;
-    for (const auto& b : bufs) { if (*b.at) cudaFree(*b.at); *b.at = nullptr; }      // no portion is in flight: every call ends with a synchronisation
-    for (const auto& b : bufs) CK(cudaMalloc(b.at, b.bytes));
-    e->pf_rows = (int)C;
+    const size_t qd = (size_t)e->q_dim_l, kd = (size_t)e->kv_dim_l;
+    struct { void** at; size_t row; } const bufs[] = {{(void**)&e->pf_x, (size_t)p.dim * 2}, {(void**)&e->pf_xn, (size_t)p.dim * 2}, {(void**)&e->pf_qkv, (qd + 2 * kd) * 4}, {(void**)&e->pf_q, qd * 2},
+                                                      {(void**)&e->pf_att, qd * 2}, {(void**)&e->pf_g, (size_t)e->inter_l * 2}, {(void**)&e->pf_tok, 4}};
+    auto bytes = [&](int r) { size_t n = 0; for (const auto& b : bufs) n += (size_t)r * b.row; return n; };
+    auto drop = [&] { for (const auto& b : bufs) { if (*b.at) cudaFree(*b.at); *b.at = nullptr; } };
+    cudaError_t why = cudaSuccess;
+    auto take = [&](int r) {
+        why = cudaStreamSynchronize(e->stream);          // a call that failed halfway may have left launches that use the old rows
+        drop();
+        for (const auto& b : bufs) if (why == cudaSuccess) why = cudaMalloc(b.at, (size_t)r * b.row);
+        if (why != cudaSuccess) drop();
+        return why == cudaSuccess;
+    };
+    e->pf_rows = portion_rows(e->pf_rows, std::min(need, kPrefillChunk), std::min(kPrefillChunk, p.max_seq_len), bytes, take);
+    if (!e->pf_rows) return fail(CUQWEN_ERR_CUDA, "no device memory for the workspace of a prompt: %s", cudaGetErrorString(why == cudaSuccess ? cudaErrorMemoryAllocation : why));
+    *rows = std::min(kPrefillChunk, e->pf_rows);
     return CUQWEN_OK;
 }
 
@@ -726,12 +735,12 @@ static int check_tokens(const cuqwen_engine* e, const int* tokens, int n_tokens,
 
 // A portion of a sequence through a layer-list design, chunk by chunk; logits of the wanted rows (ascending) to the host.
 static int stack_portion(cuqwen_engine* e, const int* tokens, int n_tokens, int pos0, const int* want, int n_want, float* logits) {
-    const int C = stack_chunk();
+    int C = 0;
     CK(cudaSetDevice(e->p.device));
-    if (int r = stack_workspace(e, std::min(n_tokens, C))) return r;
+    if (int r = stack_workspace(e, n_tokens, &C)) return r;
     if (int r = stack_begin(e->stack, pos0)) return r;
     t_err = reinterpret_cast<unsigned*>(&e->ctl->pad[0]);
-    if (!e->pf_tok) CK(cudaMalloc((void**)&e->pf_tok, (size_t)C * 4));
+    if (!e->pf_tok) CK(cudaMalloc((void**)&e->pf_tok, (size_t)stack_chunk() * 4));
     CK(cudaMemsetAsync(&e->ctl->pad[0], 0, 4, e->stream));
     CK(cudaEventRecord(e->ev0, e->stream));
     int w0 = 0;
@@ -798,8 +807,9 @@ extern "C" int cuqwen_prefill(cuqwen_engine* e, const int* tokens, int n_tokens,
     for (int i = 0; i < n_tokens; ++i) if (tokens[i] < 0 || tokens[i] >= p.vocab_size) return fail(CUQWEN_ERR_ARG, "token %d out of range", tokens[i]);
     CK(cudaSetDevice(p.device));
     t_err = reinterpret_cast<unsigned*>(&e->ctl->pad[0]);
-    const int qd = e->q_dim_l, kd = e->kv_dim_l, C = kPrefillChunk;
-    if (int r = prefill_workspace(e, std::min(n_tokens, C))) return r;
+    const int qd = e->q_dim_l, kd = e->kv_dim_l;
+    int C = 0;
+    if (int r = prefill_workspace(e, n_tokens, &C)) return r;
     const size_t kv_layer = (size_t)e->n_kv_l * p.max_seq_len * p.head_dim;
     const float eps = __half2float(__float2half(p.norm_eps));
     const int ldqkv = qd + 2 * kd;

@@ -9,6 +9,7 @@
 // Sequential layers: keys and values [kv_heads][max_seq_len][key dim | value vdim]; recurrent states float32 [heads][value channel]
 // [key channel]; the inputs that a later token still needs in rings by position.
 //   raw          [query latent q_rank | cache row | gate heads * vdim], float32 sums of the first launch of a layer
+#include "portion.h"
 #include "stack_pass.h"
 
 #include <cmath>
@@ -31,44 +32,45 @@ int stack_begin(Stack* s, int pos0) {
 }
 void stack_end(Stack* s, int pos) { s->next_pos = pos; }
 
+// Where the arrays of a workspace lie in its arena, which is there or not yet.
+static void place_ws(const Stack* s, Stack::Ws* w, int rows, bool decode) {
+    Arena2 a;
+    a.base = w->arena; a.dry = !w->arena;
+    const size_t R = (size_t)rows, E = (size_t)s->esz;
+    w->x = (float*)a.get(R * s->wp * 4);
+    w->raw = (float*)a.get(R * s->max_raw * 4);
+    w->qf = (float*)a.get(R * s->max_q * 4);
+    w->y = (float*)a.get(R * s->wp * 4);
+    w->xn1 = a.get(R * s->wp * E * s->max_var); w->xn2 = a.get(R * s->wp * E);
+    w->cq = a.get(R * s->max_qr * E); w->q = a.get(R * s->max_q * E);
+    w->att = a.get(R * s->max_att * E); w->h = a.get(R * (s->max_ff ? s->max_ff : 8) * E);
+    w->sg = a.get(R * (s->sidep ? s->sidep : 8) * E);
+    if (s->spec.recurrent()) {
+        w->z = (float*)a.get(R * s->max_z * 4); w->zin = a.get(2 * R * s->max_rank * E); w->qk = (float*)a.get(R * s->max_qk * 4); w->vv = (float*)a.get(R * s->max_vv * 4);
+        w->ro = (float*)a.get(R * s->max_ro * 4); w->att2 = a.get(R * s->max_ro * E); w->sc = (float*)a.get((R + 3) / 4 * s->max_sc * kDeltaBlock * 4); w->tail = (float*)a.get((size_t)s->wp * 4);
+        if (!decode) { w->seg_state = (float*)a.get((size_t)kTmMaxSeg * s->max_tm_state * 4); w->seg_decay = (float*)a.get((size_t)kTmMaxSeg * s->max_z * 4); }
+    }
+    if (decode) {
+        w->x2 = (float*)a.get(R * s->wp * 4);
+        w->o_lat = (float*)a.get((size_t)s->max_kvr * 4);
+        w->part_o = (float*)a.get((size_t)s->max_split * s->max_kvr * 4);
+        w->part_ml = (float*)a.get((size_t)s->max_split * s->max_heads * 8);
+    } else if (s->max_kv > 0) {
+        // keys and values of everything a portion's queries can reach: the portion and the widest window before it
+        int reach = 0;
+        for (const StLayer& l : s->layers) { const int r = l.a.window > 0 && l.a.window < s->max_seq ? l.a.window - 1 : s->max_seq; reach = r > reach ? r : reach; }
+        w->kv_rows = rows + reach < s->max_seq ? rows + reach : s->max_seq;
+        w->kv = a.get((size_t)w->kv_rows * s->max_kv * E);
+    }
+    w->bytes = a.used + 256;
+    w->rows = rows;
+}
 // The zeros (padding is read) come on the stream that the work follows on: it does not wait for the default stream.
 static int alloc_ws(cuqwen_engine* e, Stack* s, Stack::Ws* w, int rows, bool decode) {
-    Arena2 dry, real;
-    for (int pass = 0; pass < 2; ++pass) {
-        Arena2& a = pass ? real : dry;
-        const size_t R = (size_t)rows, E = (size_t)s->esz;
-        w->x = (float*)a.get(R * s->wp * 4);
-        w->raw = (float*)a.get(R * s->max_raw * 4);
-        w->qf = (float*)a.get(R * s->max_q * 4);
-        w->y = (float*)a.get(R * s->wp * 4);
-        w->xn1 = a.get(R * s->wp * E * s->max_var); w->xn2 = a.get(R * s->wp * E);
-        w->cq = a.get(R * s->max_qr * E); w->q = a.get(R * s->max_q * E);
-        w->att = a.get(R * s->max_att * E); w->h = a.get(R * (s->max_ff ? s->max_ff : 8) * E);
-        w->sg = a.get(R * (s->sidep ? s->sidep : 8) * E);
-        if (s->spec.recurrent()) {
-            w->z = (float*)a.get(R * s->max_z * 4); w->zin = a.get(2 * R * s->max_rank * E); w->qk = (float*)a.get(R * s->max_qk * 4); w->vv = (float*)a.get(R * s->max_vv * 4);
-            w->ro = (float*)a.get(R * s->max_ro * 4); w->att2 = a.get(R * s->max_ro * E); w->sc = (float*)a.get((R + 3) / 4 * s->max_sc * kDeltaBlock * 4); w->tail = (float*)a.get((size_t)s->wp * 4);
-            if (!decode) { w->seg_state = (float*)a.get((size_t)kTmMaxSeg * s->max_tm_state * 4); w->seg_decay = (float*)a.get((size_t)kTmMaxSeg * s->max_z * 4); }
-        }
-        if (decode) {
-            w->x2 = (float*)a.get(R * s->wp * 4);
-            w->o_lat = (float*)a.get((size_t)s->max_kvr * 4);
-            w->part_o = (float*)a.get((size_t)s->max_split * s->max_kvr * 4);
-            w->part_ml = (float*)a.get((size_t)s->max_split * s->max_heads * 8);
-        } else if (s->max_kv > 0) {
-            // keys and values of everything a portion's queries can reach: the portion and the widest window before it
-            int reach = 0;
-            for (const StLayer& l : s->layers) { const int r = l.a.window > 0 && l.a.window < s->max_seq ? l.a.window - 1 : s->max_seq; reach = r > reach ? r : reach; }
-            w->kv_rows = rows + reach < s->max_seq ? rows + reach : s->max_seq;
-            w->kv = a.get((size_t)w->kv_rows * s->max_kv * E);
-        }
-        if (!pass) {
-            SK(cudaMalloc((void**)&w->arena, dry.used + 256));
-            SK(cudaMemsetAsync(w->arena, 0, dry.used + 256, e->stream));
-            real.base = w->arena; real.dry = false;
-        }
-    }
-    w->rows = rows;
+    place_ws(s, w, rows, decode);
+    SK(cudaMalloc((void**)&w->arena, w->bytes));
+    SK(cudaMemsetAsync(w->arena, 0, w->bytes, e->stream));
+    place_ws(s, w, rows, decode);
     return CUQWEN_OK;
 }
 
@@ -548,24 +550,31 @@ int stack_record_step(cuqwen_engine* e, const LaunchCfg& cfg, const std::functio
     return p.head(s->dec.xn1, s->logits, 1);
 }
 
-// Workspace of a portion: rows for the longest so far, at least twice as many when it has to grow.  No portion is in flight here.
-int stack_workspace(cuqwen_engine* e, int need) {
+// Workspace of a portion: rows for the longest so far, rounded up (portion.h).
+int stack_workspace(cuqwen_engine* e, int need, int* rows) {
     Stack* s = e->stack;
     if (!s->logits_rows) {
         if (!s->xn_rows) SK(cudaMalloc((void**)&s->xn_rows, (size_t)kLogitRows * s->wp * s->esz));
         if (!s->want_rows) SK(cudaMalloc((void**)&s->want_rows, (size_t)kChunk * 4));
         SK(cudaMalloc((void**)&s->logits_rows, (size_t)kLogitRows * s->vocab_p * 4));
     }
-    if (need <= s->pf.rows) return CUQWEN_OK;
-    const int most = kChunk < s->max_seq ? kChunk : s->max_seq, rows = (need + 255) / 256 * 256, twice = 2 * s->pf.rows, want = rows > twice ? rows : twice;
-    if (s->pf.arena) SK(cudaFree(s->pf.arena));
-    s->pf = Stack::Ws{};
-    return alloc_ws(e, s, &s->pf, want < most ? want : most, false);
+    int why = CUQWEN_OK;
+    auto bytes = [&](int r) { if (!r) return (size_t)0; Stack::Ws w; place_ws(s, &w, r, false); return w.bytes; };
+    auto take = [&](int r) {
+        why = cudaStreamSynchronize(e->stream) == cudaSuccess ? CUQWEN_OK : report_error(CUQWEN_ERR_CUDA, "an earlier launch failed");      // a call that failed halfway may have left launches that use the old rows
+        if (s->pf.arena) cudaFree(s->pf.arena);
+        s->pf = Stack::Ws{};
+        if (why == CUQWEN_OK) why = alloc_ws(e, s, &s->pf, r, false);
+        if (why != CUQWEN_OK) { if (s->pf.arena) cudaFree(s->pf.arena); s->pf = Stack::Ws{}; }
+        return why == CUQWEN_OK;
+    };
+    *rows = std::min(kChunk, portion_rows(s->pf.rows, std::min(need, kChunk), std::min(kChunk, s->max_seq), bytes, take));
+    return *rows ? CUQWEN_OK : why != CUQWEN_OK ? why : report_error(CUQWEN_ERR_CUDA, "no device memory for the workspace of a portion");
 }
 
 int stack_run_chunk(cuqwen_engine* e, int T, int pos0, const int* want, int n_want, float* logits_host) {
     Stack* s = e->stack;
-    if (T < 1 || T > kChunk) return report_error(CUQWEN_ERR_ARG, "a portion has 1 to %d tokens", kChunk);
+    if (T < 1 || T > s->pf.rows) return report_error(CUQWEN_ERR_ARG, "a portion has 1 to %d tokens", s->pf.rows);
     const LaunchCfg plain{e->stream, e->sms, false}, cfg{e->stream, e->sms, !(e->p.flags & CUQWEN_FLAG_NO_PDL)};      // plain: launches that follow a copy
     Pass p{e, s, &s->pf, cfg, T, false, e->pf_tok, nullptr, pos0, nullptr};
     if (int r = p.done(launch_st_embed(s->embed.w, s->embed.pitch, e->pf_tok, s->pf.x, s->wp, s->spec.width, (float)s->spec.embed_scale, T, plain), "embedding")) return r;

@@ -27,11 +27,11 @@ void stack_end(Stack* s, int pos);
 // The launches of one decode step from the embedding to the logits, for the token / position in e->ctl.  `after` is called
 // after every launch (launch counting, profiling events).
 int stack_record_step(cuqwen_engine* e, const LaunchCfg& cfg, const std::function<int()>& after);
-int stack_workspace(cuqwen_engine* e, int rows);      // before a portion of at most `rows` tokens at a time
+int stack_workspace(cuqwen_engine* e, int need, int* rows);      // before a portion of `need` tokens; *rows: how many go through the layers together
 // A portion of a sequence: T tokens (device ids at e->pf_tok) at cache positions pos0 ..; leaves their cache rows.  Logits of
 // the rows want[0 .. n_want) (ascending row numbers of this portion) go to logits_host [n_want][vocab]; with none wanted the
-// last layer stops after its cache rows.  At most stack_chunk() tokens.
-int stack_chunk();
+// last layer stops after its cache rows.  At most as many tokens as stack_workspace answered.
+int stack_chunk();                                // the most that go through the layers together
 int stack_run_chunk(cuqwen_engine* e, int T, int pos0, const int* want, int n_want, float* logits_host);
 
 }  // namespace cq

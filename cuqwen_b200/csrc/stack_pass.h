@@ -62,7 +62,7 @@ struct Stack {
         float *z = nullptr, *qk = nullptr, *vv = nullptr, *ro = nullptr, *tail = nullptr; float *seg_state = nullptr, *seg_decay = nullptr, *sc = nullptr;      // recurrences: segments of a portion, decays, convolution outputs, read-outs, head scalars
         void *zin = nullptr, *att2 = nullptr;
         void *xn1 = nullptr, *xn2 = nullptr, *cq = nullptr, *q = nullptr, *att = nullptr, *h = nullptr, *sg = nullptr, *kv = nullptr;
-        uint8_t* arena = nullptr;
+        uint8_t* arena = nullptr; size_t bytes = 0;
     } dec, pf;
     float* dec_x = nullptr;             // where a decode step leaves the residual stream (every layer's part added)
     float* logits = nullptr;            // decode step

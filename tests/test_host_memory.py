@@ -73,3 +73,99 @@ for n in (300, 700, 4100):
     assert stub.stub_unordered() == 0, n
     at += n
 """, directories[design], act)
+
+
+OPEN = {"table": """
+def make(max_seq):
+    eng = E.Engine(E.custom_params(512, 256, 512, 2, 2, 1, 128, 2, max_seq_len=max_seq))
+    eng.load(sys.argv[1])
+    return eng
+longest = 8192
+""", "directory": """
+def make(max_seq):
+    return E.Engine.open(sys.argv[1], act=sys.argv[2], max_seq_len=max_seq)
+longest = 4096
+"""}
+ENGINES = [("table", ""), ("falivik", "bfloat16"), ("gipotar", "float32"), ("gipotar", "bfloat16")]
+
+
+@pytest.fixture(scope="module")
+def run_engine(run, directories, table_file):
+    def go(name, act, code):
+        path = table_file if name == "table" else directories[name]
+        return run(OPEN["table" if name == "table" else "directory"] + code, path, act)
+    return go
+
+
+@pytest.mark.parametrize("name,act", ENGINES)
+def test_a_prompt_is_cut_where_the_largest_workspace_does_not_fit(run_engine, name, act):
+    run_engine(name, act, """
+eng = make(9000)
+eng.prefill(toks[:256], 0)
+small = stub.stub_used()
+eng.prefill(toks[:longest], 0)
+large = stub.stub_used()
+eng.close()
+copies()
+eng = make(9000)
+eng.prefill(toks[:2], 0)                                       # 256 rows
+base = stub.stub_used()
+per_row = (large - small) / (longest - 256)
+stub.stub_limit(base + int(1500 * per_row))                    # room for some 1500 rows more than those
+copies()
+eng.prefill(toks[:5000], 0)
+cut = [n // 4 for n in copies()]
+assert sum(cut) == 5000 and 1024 <= max(cut) <= 1800 and len(cut) <= 5, cut
+eng.prefill(toks[:5000], 0)                                    # asked again: what stands does
+assert [n // 4 for n in copies()] == cut
+stub.stub_limit(1 << 40)
+eng.prefill(toks[:5000], 0)
+assert [n // 4 for n in copies()] == [min(5000, longest)] + [5000 - longest] * (longest < 5000)
+""")
+
+
+@pytest.mark.parametrize("name,act", ENGINES)
+def test_a_workspace_that_stands_is_not_given_up_for_one_that_does_not_fit(run_engine, name, act):
+    run_engine(name, act, """
+eng = make(9000)
+eng.prefill(toks[:2000], 0)
+stub.stub_limit(stub.stub_used())                              # another program holds the rest
+held = stub.stub_used()
+copies(); stub.stub_peak()
+for n in (2100, 4000, 9000):
+    eng.prefill(toks[:n], 0)
+    cut = [c // 4 for c in copies()]
+    assert sum(cut) == n and cut[0] == 2048, cut
+    assert stub.stub_used() == stub.stub_peak() == held
+""")
+
+
+@pytest.mark.parametrize("name,act", ENGINES)
+def test_a_workspace_is_no_longer_than_the_cache(run_engine, name, act):
+    run_engine(name, act, """
+eng = make(3000)
+eng.prefill(toks[:3000], 0)
+all_of_it = stub.stub_used()
+eng.close()
+eng = make(3000)
+for n in (300, 2100, 2400):
+    eng.prefill(toks[:n], 0)
+    assert stub.stub_used() <= all_of_it, n
+""")
+
+
+@pytest.mark.parametrize("name,act", ENGINES)
+def test_no_room_at_all_is_an_error_and_the_next_call_starts_clean(run_engine, name, act):
+    run_engine(name, act, """
+eng = make(3000)
+stub.stub_limit(stub.stub_used())
+try:
+    eng.prefill(toks[:700], 0)
+    raise SystemExit("a portion without a workspace")
+except CuQwenError as e:
+    assert "memory" in str(e), e
+stub.stub_limit(1 << 40)
+copies()
+eng.prefill(toks[:700], 0)
+assert [c // 4 for c in copies()] == [700]
+""")
