@@ -835,10 +835,11 @@ extern "C" int cuqwen_prefill(cuqwen_engine* e, const int* tokens, int n_tokens,
             PfAttnArgs aa; memset(&aa, 0, sizeof aa);
             aa.q = e->pf_q; aa.kc = ra.kcache; aa.vc = ra.vcache; aa.out = e->pf_att; aa.T = T; aa.pos0 = pos; aa.n_heads = e->n_heads_l;
             aa.grp = e->plan.grp; aa.max_seq = p.max_seq_len; aa.ldq = qd; aa.scale_log2 = (1.0f / sqrtf((float)p.head_dim)) * 1.4426950408889634f;
-            // Few queries near the beginning: the mma.sync kernel's short tiles are done sooner (14 heads of 64: 64 queries 4.7 against 6.2 us, 128 queries
-            // at 192 8.6 against 11.3); further on the tcgen05 kernel's longer ones pay (28 heads of 128, 64 queries: at 192 9.1 against 9.6, at 448 14.9
-            // against 13.1)
-            const bool few = T <= 128 && pos + T <= 320;
+            // The mma.sync kernel, whose tiles of 64 queries and 64 keys have the shorter chain, while every SM gets at most one of its CTAs: with heads of 64
+            // at any position (14 heads, 256 queries: from 0 on 6.2 us against 8.7 of the tcgen05 kernel, at 8000 120 against 128), with heads of 128 up
+            // to 512 keys (28 heads, 128 queries: from 0 on 5.6 against 8.2, at 320 12.3 against 13.8, at 1000 26.7 against 24.7).  With more
+            // CTAs than SMs it is behind (40 heads of 128, 256 queries from 0 on 11.5 against 10.3).
+            const bool few = e->n_heads_l * ((T + 63) / 64) <= e->sms && (p.head_dim == 64 || pos + T <= 512);
             if (!few && !(p.flags & CUQWEN_FLAG_PREFILL_ATTN_MMA)) PK(launch_prefill_attn_tc(p.head_dim, aa, e->n_kv_l, t_err, cfg));
             else PK(launch_prefill_attn(p.head_dim, aa, cfg));
             if (int r = prefill_gemm(e, PF_RESID, e->pf_att, om, 1, e->pf_x, T, p.dim)) return r;

@@ -2,7 +2,9 @@
 // the reference's decode attention (src/kernels.cu:105-288), which the reference applies once per prompt token
 // (src/main.cu:86-92).  prefill_attn.cu holds an mma.sync kernel, used for few queries near the beginning.
 //
-// One CTA = two tiles of 128 queries of one head, one CTA to an SM.  Per tile of 128 keys:
+// One CTA = two tiles of 128 queries, or one where there are SMs enough; one CTA to an SM.  The tiles of a KV group (128 queries of one of
+// its heads each) are numbered from the last queries down, the heads of the same queries side by side, and go to CTAs in that order: two tiles of a CTA
+// then mostly see the same keys, at most one CTA of a group goes without a second one, and the longest start first.  Per tile of 128 keys:
 //   warp 8      TMA: K and V tiles of the head's KV group (64-column boxes, hardware-swizzled), two slots each
 //   warp 9      one lane issues, for the two query tiles in turn, O += P V of a key tile (A = P from tensor memory, B = V as the MN-major
 //               operand straight from its cache layout) and S = Q K^T of the next (both operands K-major)
@@ -13,11 +15,15 @@
 // no barrier among the softmax warps and no pass through shared memory; what bounds it is the chain of a tile - scores, exponentials (1024
 // cycles of an SM partition's unit), P V, next scores - of which the two query tiles hide half.  Against two threads to a row, P in shared
 // memory, 64-key tiles and two CTAs to an SM: 40 heads x 8190 queries 782 us for 999 (0.88 PFLOP/s), 16 heads x 3000 queries at 1000 115 for 140.
+// Two tiles of one head to every CTA left SMs idle where there are few, and half of the last CTAs idle: 40 heads x 777 queries at 3000 135 us, now 76;
+// 28 heads x 192 from 0 on 11.3, now 8.7; 14 heads of 64 x 512 at 1000 31.3, now 27.7 (64-key tiles, two CTAs to an SM: 92, 7.7 and 27.0).
 // The tensor core finishes its MMAs in the order of issue: when S of a key tile is there, so is P V of the one before, and O may be rescaled.
 // Every mbarrier wait is bounded; a wait that runs out sets *err and the CTA drains.
 #include "prefill.cuh"
 #include "stack_dev.cuh"
 #include "tcgen05.cuh"
+
+#include <algorithm>
 
 namespace cq {
 
@@ -28,15 +34,16 @@ constexpr int kTaThreads = 320;
 constexpr int kTaBlk = 128 * 128;
 __host__ __device__ constexpr int ta_tile(int hd) { return hd / 64 * kTaBlk; }
 __host__ __device__ constexpr int ta_smem(int hd) { return 6 * ta_tile(hd) + 256; }
-// TMEM columns: S (128; P in the first 64 of them) and O (HD, 128 at the most) of one query tile or two.  A launch of at most 128 queries takes
+// TMEM columns: S (128; P in the first 64 of them) and O (HD, 128 at the most) of one query tile or two.  A launch without pairs takes
 // half of the memory, so that the next launch's first CTAs find some.
-__host__ __device__ constexpr uint32_t ta_cols(int T) { return T > kTaBM ? 512u : 256u; }
+__host__ __device__ constexpr uint32_t ta_cols(bool pairs) { return pairs ? 512u : 256u; }
 
 struct PfAttnTcArgs {
     CUtensorMap tq;          // q as [T][ldq] fp16, box 64 x 128, swizzled
     CUtensorMap tk, tv;      // caches as [n_kv][rows][hd] fp16, box 64 x 128 x 1, swizzled
     __half* out;
-    int T, pos0, n_heads, grp, ldq;
+    int T, pos0, n_kv, grp, ldq;
+    int singles;             // query tiles of a KV group, from the longest down, that have a CTA to themselves
     float scale_log2;
     unsigned* err;
 };
@@ -51,13 +58,17 @@ __global__ void __launch_bounds__(kTaThreads, 1) prefill_attn_tc_kernel(const __
     const uint32_t sQ = base, sK = sQ + 2 * kTile, sV = sK + 2 * kTile, bars = sV + 2 * kTile;
     const uint32_t b_q = bars, b_kfull = bars + 8, b_kfree = bars + 24, b_vfull = bars + 40, b_vfree = bars + 56, b_s = bars + 72, b_p = bars + 88, b_o = bars + 120, tmem_slot = bars + 136;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int head = blockIdx.y, kvh = head / a.grp;
-    const int q0 = (gridDim.x - 1 - blockIdx.x) * (kTaQ * kTaBM);         // the longest tiles first
-    const int nq = q0 + kTaBM < a.T ? 2 : 1;                             // query tiles that have queries
-    auto key_end = [&](int i) { return a.pos0 + min(q0 + (i + 1) * kTaBM, a.T); };      // keys that query tile i sees at all
-    auto tiles = [&](int i) { return (key_end(i) + kTaBN - 1) / kTaBN; };               // its key tiles; the last query tile has the most
+    const int kvh = blockIdx.x % a.n_kv, cta = blockIdx.x / a.n_kv, nqt = (a.T + kTaBM - 1) / kTaBM, units = nqt * a.grp;
+    const int u0 = cta < a.singles ? cta : 2 * cta - a.singles;
+    const int nq = cta >= a.singles && u0 + 1 < units ? 2 : 1;            // query tiles of this CTA; the last one sees the most keys
+    const int qlast = (nqt - 1 - u0 / a.grp) * kTaBM, hlast = kvh * a.grp + u0 % a.grp;
+    const int qfirst = nq > 1 ? (nqt - 1 - (u0 + 1) / a.grp) * kTaBM : qlast, hfirst = nq > 1 ? kvh * a.grp + (u0 + 1) % a.grp : hlast;
+    auto q0 = [&](int i) { return i == nq - 1 ? qlast : qfirst; };        // tile i: first query, head
+    auto head = [&](int i) { return i == nq - 1 ? hlast : hfirst; };
+    auto key_end = [&](int i) { return a.pos0 + min(q0(i) + kTaBM, a.T); };             // keys that it sees at all
+    auto tiles = [&](int i) { return (key_end(i) + kTaBN - 1) / kTaBN; };
     const int nj = tiles(nq - 1);
-    const uint32_t cols = ta_cols(a.T);
+    const uint32_t cols = ta_cols(a.singles < units);
     bool failed = false;
 
     if (threadIdx.x == 256) { prefetch_map(&a.tq); prefetch_map(&a.tk); prefetch_map(&a.tv); }
@@ -82,7 +93,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) prefill_attn_tc_kernel(const __
             pdl_wait();           // everything below follows from these loads
             mbar_expect_tx(b_q, (uint32_t)(nq * kTile));
             for (int i = 0; i < nq; ++i)
-                for (int b = 0; b < NBLK; ++b) tma_load_2d(sQ + i * kTile + b * kTaBlk, &a.tq, head * HD + 64 * b, q0 + i * kTaBM, b_q);
+                for (int b = 0; b < NBLK; ++b) tma_load_2d(sQ + i * kTile + b * kTaBlk, &a.tq, head(i) * HD + 64 * b, q0(i), b_q);
             for (int j = 0; j < nj; ++j) {
                 const int s = j & 1; const uint32_t free_par = (((uint32_t)j >> 1) & 1u) ^ 1u;
                 if (!mbar_wait(b_kfree + 8 * s, free_par)) { failed = true; break; }
@@ -136,7 +147,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) prefill_attn_tc_kernel(const __
         }
     } else if ((warp >> 2) < nq) {
         const int i = warp >> 2, r = (warp & 3) * 32 + lane;              // query tile, row of it = TMEM lane
-        const int qpos = a.pos0 + q0 + i * kTaBM + r, mine = tiles(i);
+        const int qi = q0(i), qpos = a.pos0 + qi + r, mine = tiles(i);
         const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16, s_at = tS + (uint32_t)(i * kTaBN) + lane_off, o_at = tO + (uint32_t)(i * HD) + lane_off;
         // m is the exponent the row's probabilities are scaled by, not always its running maximum: it moves only when
         // a tile's maximum exceeds it by more than 2^8 (probabilities then stay below 256, well inside fp16, and the
@@ -157,7 +168,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) prefill_attn_tc_kernel(const __
                 mx4[c] = -INFINITY;
                 if (c >= nc) continue;
                 const int key = key0 + c * 32;
-                if (key + 31 > a.pos0 + q0 + i * kTaBM) {                 // some key of this piece may lie past some query (uniform over the tile)
+                if (key + 31 > a.pos0 + qi) {                 // some key of this piece may lie past some query (uniform over the tile)
 #pragma unroll
                     for (int k = 0; k < 32; ++k) if (key + k > qpos) x[c][k] = 0xff800000u;      // -infinity
                 }
@@ -208,13 +219,13 @@ __global__ void __launch_bounds__(kTaThreads, 1) prefill_attn_tc_kernel(const __
         if (!failed && !mbar_wait(b_o + 8 * i, 0u)) failed = true;
         tc_fence_after();
         const float inv = 1.0f / l;
-        const int t = q0 + i * kTaBM + r;
+        const int t = qi + r;
 #pragma unroll 1
         for (int c = 0; c < HD / 32; ++c) {
             float v[32];
             tmem_ld32(o_at + (uint32_t)(c * 32), v);
             if (t < a.T && !failed) {
-                __half* dst = a.out + (size_t)t * a.ldq + head * HD + c * 32;
+                __half* dst = a.out + (size_t)t * a.ldq + head(i) * HD + c * 32;
 #pragma unroll
                 for (int k = 0; k < 32; k += 8)
                     *reinterpret_cast<uint4*>(dst + k) = make_uint4(pack_h2(v[k] * inv, v[k + 1] * inv), pack_h2(v[k + 2] * inv, v[k + 3] * inv),
@@ -256,7 +267,7 @@ static int ta_go(const PfAttnTcArgs& k, dim3 grid, const LaunchCfg& cfg) {
 int launch_prefill_attn_tc(int head_dim, const PfAttnArgs& a, int n_kv, unsigned* err, const LaunchCfg& cfg) {
     const int kTaHD = head_dim;
     if (head_dim != 64 && head_dim != 128) return (int)cudaErrorInvalidValue;
-    if (a.T <= 0 || a.pos0 < 0 || a.pos0 + a.T > a.max_seq || a.n_heads <= 0 || a.grp <= 0 || a.ldq % 8 || n_kv <= 0) return (int)cudaErrorInvalidValue;
+    if (a.T <= 0 || a.pos0 < 0 || a.pos0 + a.T > a.max_seq || a.grp <= 0 || a.ldq % 8 || n_kv <= 0 || a.n_heads != n_kv * a.grp) return (int)cudaErrorInvalidValue;
     TaEncodeFn fn = ta_encode();
     if (!fn) return (int)cudaErrorNotSupported;
     PfAttnTcArgs k; memset(&k, 0, sizeof k);
@@ -276,8 +287,13 @@ int launch_prefill_attn_tc(int head_dim, const PfAttnArgs& a, int n_kv, unsigned
         if (fn(maps[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half*>(caches[i]), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return (int)cudaErrorInvalidValue;
     }
-    k.out = a.out; k.T = a.T; k.pos0 = a.pos0; k.n_heads = a.n_heads; k.grp = a.grp; k.ldq = a.ldq; k.scale_log2 = a.scale_log2; k.err = err;
-    const dim3 grid((a.T + kTaQ * kTaBM - 1) / (kTaQ * kTaBM), a.n_heads);
+    k.out = a.out; k.T = a.T; k.pos0 = a.pos0; k.n_kv = n_kv; k.grp = a.grp; k.ldq = a.ldq; k.scale_log2 = a.scale_log2; k.err = err;
+    const int units = (a.T + kTaBM - 1) / kTaBM * a.grp;
+    // Alone a tile is done sooner (14 heads of 64, 129 queries at 8000: 126 us for 136 in pairs): as many as leave no CTA without an SM, and none
+    // with more than two tiles to an SM.
+    const int slots = cfg.sm_count / n_kv;
+    k.singles = std::min(units, std::max(0, 2 * slots - units));
+    const dim3 grid((k.singles + (units - k.singles + 1) / 2) * n_kv);
     return head_dim == 128 ? ta_go<128>(k, grid, cfg) : ta_go<64>(k, grid, cfg);
 }
 

@@ -1,6 +1,6 @@
 // A CUDA runtime without a GPU, preloaded before libcudart: device memory is host memory under a limit, copies and fills happen at once,
 // kernels do nothing.  It serves tests of host logic: which memory a call takes, how a prompt is cut, and whether work on a stream may run before a fill that
-// was queued on the default stream.
+// was queued on the default stream, and which kernels with which grids a call launches.
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -18,6 +18,9 @@ static std::map<char*, size_t> filled;                 // written on the default
 static size_t limit = (size_t)1 << 40, used = 0, peak = 0;
 static long unordered = 0;
 static std::string copies;                             // bytes of every host-to-device copy on a stream
+static std::map<const void*, std::string> kernels;     // host stub -> name of the kernel
+static std::string launches;                           // name gx,gy,gz cluster-x,y,z, a line a launch
+static int sms = 148;
 static cudaError_t last = cudaSuccess;
 
 static size_t device_range(const void* p, char** base) {
@@ -30,6 +33,13 @@ static size_t device_range(const void* p, char** base) {
 }
 // Work is queued on a stream that does not wait for the default one: every block that a fill may still be writing counts.
 static void work_on(cudaStream_t s) { if (s) unordered += (long)filled.size(); }
+static void launched(const void* f, dim3 g, dim3 c, cudaStream_t s) {
+    std::lock_guard<std::mutex> lk(mu);
+    work_on(s);
+    char at[96];
+    snprintf(at, sizeof at, " %u,%u,%u %u,%u,%u\n", g.x, g.y, g.z, c.x, c.y, c.z);
+    launches += kernels[f] + at;
+}
 static cudaError_t err(cudaError_t e) { if (e != cudaSuccess) last = e; return e; }
 
 extern "C" {
@@ -38,6 +48,8 @@ void stub_limit(size_t bytes) { limit = bytes; }
 size_t stub_used() { return used; }
 size_t stub_peak() { const size_t p = peak; peak = used; return p; }
 long stub_unordered() { const long n = unordered; unordered = 0; return n; }
+void stub_sms(int n) { sms = n; }
+const char* stub_launches() { static std::string out; out = launches; launches.clear(); return out.c_str(); }
 const char* stub_copies() { static std::string out; out = copies; copies.clear(); return out.c_str(); }
 
 // ---- memory
@@ -88,7 +100,7 @@ cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size
 // ---- device, streams, events
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
-cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 148; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = sms; return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() { std::lock_guard<std::mutex> lk(mu); filled.clear(); return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStream_t)malloc(8); return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { free(s); return cudaSuccess; }
@@ -107,8 +119,22 @@ cudaError_t cudaPeekAtLastError() { return last; }
 
 // ---- kernels
 cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
-cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t s) { std::lock_guard<std::mutex> lk(mu); work_on(s); return cudaSuccess; }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void*, void**) { std::lock_guard<std::mutex> lk(mu); work_on(c->stream); return cudaSuccess; }
+cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3, void**, size_t, cudaStream_t s) { launched(f, g, dim3(1, 1, 1), s); return cudaSuccess; }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
+    dim3 cl(1, 1, 1);
+    for (unsigned i = 0; i < c->numAttrs; ++i)
+        if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) cl = dim3(c->attrs[i].val.clusterDim.x, c->attrs[i].val.clusterDim.y, c->attrs[i].val.clusterDim.z);
+    launched(f, c->gridDim, cl, c->stream);
+    return cudaSuccess;
+}
+void** __cudaRegisterFatBinary(void*) { static void* handle[1]; return handle; }
+void __cudaRegisterFatBinaryEnd(void**) {}
+void __cudaUnregisterFatBinary(void**) {}
+void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
+void __cudaRegisterFunction(void**, const char* host, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*) { kernels[host] = name; }
+static thread_local struct { dim3 g, b; size_t smem; void* s; } config;      // between the two halves of kernel<<<>>>()
+unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t smem, void* s) { config = {g, b, smem, s}; return 0; }
+cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* smem, void* s) { *g = config.g; *b = config.b; *smem = config.smem; *(void**)s = config.s; return cudaSuccess; }
 static CUresult encode(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                        CUtensorMapL2promotion, CUtensorMapFloatOOBfill) { return CUDA_SUCCESS; }
 cudaError_t cudaGetDriverEntryPoint(const char* name, void** f, unsigned long long, cudaDriverEntryPointQueryResult* q) {

@@ -338,6 +338,15 @@ def test_prefill_attention_at_tile_edges(built, hd, T, pos0, nh, nkv):
     test_prefill_attention_kernels(built, 0, hd, T, pos0, nh, nkv)
 
 
+# more tiles than SMs: pairs of one head's query tiles (a head to a KV group), of two heads with the same queries, with neighbouring ones, an odd number
+# of tiles in a group, and the longest tiles alone beside pairs of the others
+@pytest.mark.parametrize("hd", [128, 64])
+@pytest.mark.parametrize("T,pos0,nh,nkv", [(129, 0, 150, 150), (255, 3, 150, 150), (256, 0, 149, 149), (257, 127, 150, 150), (385, 0, 150, 150), (100, 0, 228, 76), (200, 60, 228, 76), (128, 1, 300, 150),
+                                           (640, 0, 40, 8), (777, 100, 40, 8), (1024, 0, 40, 8)])
+def test_prefill_attention_with_pairs_of_query_tiles(built, hd, T, pos0, nh, nkv):
+    test_prefill_attention_kernels(built, 0, hd, T, pos0, nh, nkv)
+
+
 @pytest.mark.parametrize("hd", [128, 64])
 def test_prefill_attention_moves_its_exponent(built, hd):
     """Scores that grow from key tile to key tile by far more than 2^8, so that every tile rescales what has been summed."""

@@ -24,7 +24,7 @@ stub = ctypes.CDLL(os.environ["LD_PRELOAD"])
 stub.stub_limit.argtypes = [ctypes.c_size_t]
 stub.stub_used.restype = stub.stub_peak.restype = ctypes.c_size_t
 stub.stub_unordered.restype = ctypes.c_long
-stub.stub_copies.restype = ctypes.c_char_p
+stub.stub_copies.restype = stub.stub_launches.restype = ctypes.c_char_p
 copies = lambda: [int(n) for n in stub.stub_copies().split()]
 toks = np.arange(20000, dtype=np.int32) % 50
 """

@@ -1,0 +1,27 @@
+"""Which kernels a call launches, on the CPU over tests/cudart_stub.cpp."""
+import pytest
+
+from cuqwen_b200 import binfmt
+from test_host_memory import run                                           # noqa: F401  (fixture)
+
+
+@pytest.mark.parametrize("hd,sms,sizes", [
+    # (tokens, position) -> the mma.sync kernel, else the tcgen05 one; two heads
+    (128, 148, [(1, 0, True), (512, 0, True), (513, 0, False), (100, 412, True), (100, 413, False), (1, 9000, False)]),
+    (64, 148, [(1, 0, True), (4736, 0, True), (4737, 0, False), (64, 9000, True)]),
+    (64, 7, [(192, 0, True), (193, 0, False), (64, 9000, True)]),
+])
+def test_attention_kernel_of_a_prompt(run, tmp_path, hd, sms, sizes):      # noqa: F811
+    cfg = dict(vocab=512, dim=256, inter=512, layers=2, heads=2, kv=1, hd=hd, tied=True)
+    path = tmp_path / "m.bin"
+    binfmt.write_model(path, cfg, 2, binfmt.random_tensors(cfg, 3))
+    run(f"""
+stub.stub_sms({sms})
+eng = E.Engine(E.custom_params(512, 256, 512, 2, 2, 1, {hd}, 2, max_seq_len=10000))
+eng.load(sys.argv[1])
+for n, pos, mma in {sizes}:
+    stub.stub_launches()
+    eng.prefill(toks[:n], pos)
+    names = stub.stub_launches().decode()
+    assert ("prefill_attn_kernel" in names, "prefill_attn_tc_kernel" in names) == (mma, not mma), (n, pos, names)
+""", path)
