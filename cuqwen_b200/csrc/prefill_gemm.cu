@@ -466,7 +466,7 @@ static int pf_row_tiles(const int* rows, int nmat, bool swiglu, int nt) {
 
 // SMs that clusters of n CTAs (one CTA to an SM) can fill at once: a cluster lies within one GPU processing cluster, so sizes of
 // four and eight leave some over (measured on 148 SMs: 33 clusters of four run side by side and 36 do not, 14 of eight and 16 not).
-static int pf_room(int n, int sms) { return n <= 2 ? sms : n == 4 ? sms * 132 / 148 : sms * 112 / 148; }
+static int pf_room(int n, int sms) { return std::max(1, n <= 2 ? sms : n == 4 ? sms * 132 / 148 : sms * 112 / 148); }
 
 // Tile and split of a product, by an estimate in SM cycles: waves of CTAs, each a fixed part (barriers, tensor memory, first
 // copies, epilogue) and a part per K block (the largest of its MMAs, its bytes through shared memory at 128 a cycle and its bytes

@@ -25,3 +25,29 @@ for n, pos, mma in {sizes}:
     names = stub.stub_launches().decode()
     assert ("prefill_attn_kernel" in names, "prefill_attn_tc_kernel" in names) == (mma, not mma), (n, pos, names)
 """, path)
+
+
+PLAN_OF = """
+import re
+from cuqwen_b200 import binfmt
+from cuqwen_b200 import kernels as K
+def plan(quant, kind, tokens, rows, cols):
+    stub.stub_launches()
+    s = 4096 if quant else None
+    if quant == 3: K.linear(0, K.LIN_F32, 4096, cols, 4096, -(-cols // 128) * 128, cols, tokens, rows, 4096, rows)
+    elif kind == "swiglu": K.prefill_gemm(quant, K.PF_SWIGLU, 4096, 4096, s, 4096, tokens, rows, cols, w1=4096, s1=s)
+    else: K.prefill_gemm(quant, K.PF_RESID, 4096, 4096, s, 4096, tokens, rows, cols)
+    name, _, cluster = stub.stub_launches().decode().split()
+    return tuple(int(v) for v in re.search("prefill_gemm_kernelILi.ELi(\\d+)ELi(\\d+)ELi(\\d+)E", name).groups()) + (int(cluster.split(",")[2]),)
+"""
+
+
+def test_a_plan_on_any_number_of_sms(run):                                 # noqa: F811
+    """Down to one SM, of which no cluster of four fits any."""
+    run(PLAN_OF + """
+for sms in (0, 1, 2, 3, 7, 20, 74, 132, 148, 160):
+    stub.stub_sms(sms)
+    for size in ((5, 72, 2048), (61, 896, 4864), (700, 6408, 256), (4096, 1536, 1536)):
+        for quant in range(4):
+            assert plan(quant, "plain", *size)[0] in (64, 128, 192, 224, 256)
+""")
