@@ -488,12 +488,14 @@ constexpr int kGemvThreadsHost = (kConsumerWarps + 1) * 32;
 // 5.1: sixteen consumer warps per SM, and the SMs with one block leave their share of the bandwidth to the others.
 // Everywhere else an SM holds one CTA (its shared memory, or the registers of a two-matrix kernel), blocks go round by round, and a last round
 // that is nearly empty lasts as long as a full one: 4864 rows as 152 blocks of 32 on 148 SMs took a second round for four of them.
-// There the block may have any multiple of eight rows (the scales of a block begin on 16 bytes), if that shortens rounds x rows by a
-// twentieth or more; a block of fewer rows than its row-warps cover idles some of the eight warps.  (Step of the 0.5B int4 model 722 -> 679 us,
-// of six 14B int8 layers 721 -> 685 us.  With many rounds the SMs that are ahead take the memory's rate over: lm_head, nine
-// rounds of 128 rows, was 3 to 7 % slower as nine of 120.)
+// There the block may have any multiple of eight rows (the scales of a block begin on 16 bytes), if that shortens rounds x rows enough; a block of fewer
+// rows than its row-warps cover idles some of the eight warps.  (Step of the 0.5B int4 model 722 -> 679 us, of six 14B int8 layers
+// 721 -> 685 us.)  Enough, for int8 and fp16, depends on the bytes of a whole block, measured over 27 row counts x 5 column counts: below 100 KB
+// rounds are latency, and a tenth will do (int8 add 7168 x 896 4.6 -> 4.1 us); around what a CTA's ring holds, 220 KB, both rounds'
+// copies are under way at once, and a third is needed (fp16 add 6912 x 3584: 8.5 us in 216 blocks of 32, 9.8 in 144 of 48; 5120 x 3584 8.6 in
+// 160, 8.1 in 128 of 40); above 300 KB a sixth (int8 gate/up 13,824 x 5120 27.0 -> 24.9).
+// With many rounds the SMs that are ahead take the memory's rate over: lm_head, nine rounds of 128 rows, was 3 to 7 % slower as nine of 120.
 int gemv_block_rows(int rows, int K, int sm_count, int epi, int quant) {
-    (void)K;
     if (epi == EPI_QKV) return 16;
     const int nsets = (rows + 15) / 16;
     int rw = 1;
@@ -502,9 +504,12 @@ int gemv_block_rows(int rows, int K, int sm_count, int epi, int quant) {
     if (sm_count <= 0 || (quant == Q_I4 && epi != EPI_SWIGLU)) return whole;
     auto rounds = [&](int b) { return ((rows + b - 1) / b + sm_count - 1) / sm_count; };
     if (rounds(whole) > 3) return whole;
-    int best = whole, cost = rounds(whole) * whole;
+    const long bytes = (long)whole * K * (quant == Q_F16 ? 4 : quant == Q_I8 ? 2 : 1) / 2 * (epi == EPI_SWIGLU ? 2 : 1);
+    const double enough = quant == Q_I4 ? 0.95 : bytes < 100 << 10 ? 0.9 : bytes < 300 << 10 ? 2.0 / 3 : 5.0 / 6;
+    int best = whole;
+    const double most = enough * (rounds(whole) * whole) + 1e-6;
     for (int b = 128; b > whole / 2 && b >= 24; b -= 8)
-        if (20 * rounds(b) * b <= 19 * cost && (best == whole || rounds(b) * b < rounds(best) * best)) best = b;
+        if (rounds(b) * b <= most && (best == whole || rounds(b) * b < rounds(best) * best)) best = b;
     return best;
 }
 

@@ -27,6 +27,26 @@ for n, pos, mma in {sizes}:
 """, path)
 
 
+def test_blocks_of_a_decode_product(run):                                  # noqa: F811
+    """CTAs of a GEMV: blocks that end in one round where that was measured to pay, whole tiles (then every SM has a CTA) elsewhere."""
+    run("""
+from cuqwen_b200 import kernels as K
+def grid(quant, rows, cols, gate_up):
+    stub.stub_launches()
+    s = 4096 if quant else None
+    if gate_up: K.fused_mlp_stage1(quant, 4096, 4096, 4096, s, s, 4096, cols, rows)
+    else: K.gemv_add(quant, 4096, s, 4096, 4096, rows, cols)
+    name, grid, _ = stub.stub_launches().decode().split()
+    assert "gemv_kernel" in name
+    return int(grid.split(",")[0])
+for quant, rows, cols, gate_up, ctas in [(1, 7168, 896, False, 128), (1, 4864, 896, True, 122), (2, 4864, 896, True, 122), (2, 11008, 2048, True, 138),      # blocks below 100 KB, int4
+                                         (0, 5120, 3584, False, 128), (1, 11008, 2048, True, 138), (0, 6912, 3584, False, 148), (1, 8192, 3584, True, 148),   # about a ring
+                                         (0, 27648, 896, False, 148), (1, 13824, 1536, True, 148),
+                                         (1, 13824, 5120, True, 144), (0, 13824, 3584, False, 144), (0, 8192, 5120, False, 148)]:                            # several rings
+    assert grid(quant, rows, cols, gate_up) == ctas, (quant, rows, cols, gate_up, grid(quant, rows, cols, gate_up), ctas)
+""")
+
+
 PLAN_OF = """
 import re
 from cuqwen_b200 import binfmt
