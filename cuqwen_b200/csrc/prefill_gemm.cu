@@ -4,6 +4,7 @@
 #include "tcgen05.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace cq {
 
@@ -468,10 +469,13 @@ static int pf_row_tiles(const int* rows, int nmat, bool swiglu, int nt) {
 // four and eight leave some over (measured on 148 SMs: 33 clusters of four run side by side and 36 do not, 14 of eight and 16 not).
 static int pf_room(int n, int sms) { return std::max(1, n <= 2 ? sms : n == 4 ? sms * 132 / 148 : sms * 112 / 148); }
 
-// Tile and split of a product, by an estimate in SM cycles: waves of CTAs, each a fixed part (barriers, tensor memory, first
-// copies, epilogue) and a part per K block (the largest of its MMAs, its bytes through shared memory at 128 a cycle and its bytes
-// from L2 at 56), and for a split the exchange of partial sums.  Against the fastest of all shapes, over fp16, int8, int4 and bfloat16
-// matrices of four models and 61 to 4096 tokens, the choice is within 5 % in most cases and within 35 % in all.  What the lines are about:
+// Tile and split of a product, by an estimate: waves of CTAs, each a fixed part and a part per K block (the largest of its MMAs, its bytes through
+// shared memory and its widening), and for a split the exchange of partial sums.  The constants began as SM cycles and are fitted to
+// measurements of every legal shape and split: the products of five models and two layer-list designs at 8 to 8191 tokens in fp16, int8,
+// int4 and bfloat16, 1250 products.  The fit makes a wave dear (the fixed part is some 30,000 whatever the K), and a partly filled last one nearly as dear
+// as a full one.  Over those products the choice is 0.9 % slower than the fastest shape on average, more than 10 % slower for 29
+// of them and at the most 25 %; over 210 products of random sizes 1.4 %, 10 and 26 %.  (With the constants as they had been derived: 3.2 %, 157 and
+// 49 %; 2.3 %, 21 and 33 %.)  What the lines are about:
 //   few tiles  a split of K over a cluster: 61 tokens x [896 x 4864] int8 38 us in 14 tiles, 12 in 14 clusters of eight; 500 tokens x
 //              [3584 x 18944] int4 151 us with 64-row tiles, 81 with 256 x 256 tiles in clusters of four
 //   many       pairs, and the width that fills the last wave: 2048 tokens x [3584 x 3584] int4 53 us with single CTAs, 46 with pairs of 224
@@ -485,13 +489,13 @@ static PfPlan pf_plan(int quant, int T, const int* rows, int nmat, bool swiglu, 
         if ((mh * cg > 1 && T <= kPfM) || (mh * cg > 2 && T <= 2 * kPfM) || (swiglu && nt % 64)) continue;
         const int tok = kPfM * mh * cg, ctas = (T + tok - 1) / tok * pf_row_tiles(rows, nmat, swiglu, nt) * cg;
         const double raw = pf_raw_bytes(quant, br), xb = mh * kPfABytes, bb = br * 128;
-        const double smem = (xb + 2 * raw + bb + mh * (kPfABytes + bb)) / 128, l2 = (xb + (raw > 0 ? raw : bb)) / 56;
-        const double kcyc = std::max(std::max(2.0 * mh * nt, smem), std::max(l2, 300.0));
+        const double smem = (xb + 2 * raw + bb + mh * (kPfABytes + bb)) / 136, widen = quant == Q_I4 ? 3.65 * br : quant == Q_I8 ? 4.0 * br : 0.0;
+        const double kcyc = std::max(std::max(2.25 * mh * nt, smem), std::max(widen, 460.0)) + (cg == 2 ? 70.0 : 0.0);
         const int kstep = pf_widens(quant) ? 2 : 1, nku = nkb / kstep, units = 4 * mh * nt / (swiglu ? 64 : 32);
         for (int s = 1; s <= (cg == 2 ? 1 : 8) && s <= nku; s *= 2) {
             if (units % s || (mh == 2 && nt == 256 && s > 4)) break;
-            const int room = pf_room(s, sms), waves = (ctas * s + room - 1) / room;
-            const double t = waves * (3000.0 + 8.0 * mh * nt + (double)((nku + s - 1) / s) * kstep * kcyc) + (s > 1 ? 1500.0 + 16.0 * mh * nt * (s - 1) / s : 0.0);
+            const double fill = (double)ctas * s / pf_room(s, sms), full = std::ceil(fill), waves = full > 1 ? full - 0.13 * (full - fill) : full;
+            const double t = waves * (30000.0 + 7.0 * mh * nt + (double)((nku + s - 1) / s) * kstep * kcyc) + (s > 1 ? 1400.0 + 14.0 * mh * nt * (s - 1) / s : 0.0);
             if (t < best_t) { best_t = t; best = PfPlan{nt, mh, s, cg}; }
         }
     }

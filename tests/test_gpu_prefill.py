@@ -8,6 +8,7 @@ import pytest
 
 from cuqwen_b200 import binfmt
 from cuqwen_b200 import kernels as K
+from gemm_plans import cases
 from tests.gpu_util import DevBuf, close, dev, quant_mats, report, sync
 
 pytestmark = pytest.mark.gpu
@@ -21,8 +22,7 @@ def dequant(w, s, quant, cols):
 
 
 @pytest.mark.parametrize("quant", [2, 1, 0])
-# the launcher takes 64- or 128-row tiles while 256-row tiles would fill less than a quarter / half of the SMs: the last
-# two cases are wide enough for 128 and for 256
+# token and row counts that end inside a tile, and whole ones
 @pytest.mark.parametrize("T,R,Kc", [(1, 256, 128), (37, 512, 896), (128, 576, 3584), (300, 1024, 1536), (257, 264, 256), (300, 6408, 256), (600, 6408, 256)])
 def test_prefill_gemm_plain_modes(built, quant, T, R, Kc):
     rng = np.random.default_rng(T * 131 + R + quant)
@@ -73,8 +73,7 @@ def test_prefill_gemm_swiglu(built, quant, T, R, Kc):
     assert close(got, want), report(got, want)
 
 
-# Every tile shape and split that the launcher's rule chooses, each at a size with ragged tokens and rows: splits of K over two, four and
-# eight CTAs, pairs of CTAs with 128, 192, 224 and 256 rows, one and two token halves.
+# ragged tokens and rows around the tiles' sizes, few columns and many
 @pytest.mark.parametrize("quant", [2, 1, 0])
 @pytest.mark.parametrize("T,R,Kc", [(1, 72, 640), (5, 72, 2048), (37, 2312, 2048), (61, 6408, 2048), (61, 6408, 3072), (33, 904, 3072), (129, 6408, 256), (257, 6408, 256), (257, 8200, 256),
                                     (513, 3080, 256), (513, 6408, 256), (513, 8200, 256), (700, 6408, 256), (1025, 6408, 256), (500, 1800, 3072)])
@@ -101,6 +100,17 @@ def test_prefill_gemm_swiglu_tiles_and_splits(built, quant, T, R, Kc):
     e = [6 * 2.0 ** -11 / 3 ** 0.5 * np.sqrt((xf * xf) @ (d * d).T) for d in (dg, du)]
     lim = 1.1 * np.abs(u) * e[0] + np.abs(silu) * e[1] + e[0] * e[1] + 2.0 ** -10 * np.abs(silu * u) + 1e-4
     assert (np.abs(got - silu * u) <= lim).all(), report(got, silu * u)
+
+
+@pytest.mark.parametrize("quant,kind,plan,T,R,Kc", cases((2, "plain"), (1, "plain"), (0, "plain")))
+def test_prefill_gemm_under_every_plan(built, quant, kind, plan, T, R, Kc):
+    """Every tile shape and split that the launcher's rule chooses for a model (gemm_plans.py), each at a size with ragged tokens and rows."""
+    test_prefill_gemm_plain_modes(built, quant, T, R, Kc)
+
+
+@pytest.mark.parametrize("quant,kind,plan,T,R,Kc", cases((2, "swiglu"), (1, "swiglu"), (0, "swiglu")))
+def test_prefill_gemm_swiglu_under_every_plan(built, quant, kind, plan, T, R, Kc):
+    test_prefill_gemm_swiglu_tiles_and_splits(built, quant, T, R, Kc)
 
 
 CFGS = {

@@ -14,6 +14,7 @@ import pytest
 from cuqwen_b200 import CuQwenError
 from cuqwen_b200 import engine as E
 from cuqwen_b200 import kernels as K
+from gemm_plans import cases
 from gpu_util import Pool, dev
 from stack_util import F, L, check, errors, odd, run_portions, small, tiles, weights
 
@@ -84,10 +85,16 @@ def test_linear(built, act, n, rows, cols, cols2):
         near(read_act(out, "float32" if f32 else act, (n, rows)), want, "float32" if f32 else act)
 
 
-# tiles and splits of the tensor-core GEMM that the sizes above do not reach (with and without a second product)
+# larger products, with and without a second one
 @pytest.mark.parametrize("n,rows,cols,cols2", [(33, 904, 2048, 1024), (61, 6408, 1000, 520), (129, 6408, 256, 0), (257, 8200, 200, 72), (513, 8200, 256, 0), (700, 6408, 192, 64), (1025, 6408, 256, 0)])
 def test_linear_tiles_and_splits(built, n, rows, cols, cols2):
     test_linear(built, "bfloat16", n, rows, cols, cols2)
+
+
+@pytest.mark.parametrize("quant,kind,plan,n,rows,cols", cases((3, "plain")))
+def test_linear_under_every_plan(built, quant, kind, plan, n, rows, cols):
+    """Every tile shape and split of the tensor-core GEMM that the launcher's rule chooses for a design (gemm_plans.py)."""
+    test_linear(built, "bfloat16", n, rows, cols, 0)
 
 
 @pytest.mark.parametrize("act", ACTS)

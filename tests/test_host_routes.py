@@ -2,6 +2,7 @@
 import pytest
 
 from cuqwen_b200 import binfmt
+from gemm_plans import PLANS
 from test_host_memory import run                                           # noqa: F401  (fixture)
 
 
@@ -60,6 +61,32 @@ def plan(quant, kind, tokens, rows, cols):
     name, _, cluster = stub.stub_launches().decode().split()
     return tuple(int(v) for v in re.search("prefill_gemm_kernelILi.ELi(\\d+)ELi(\\d+)ELi(\\d+)E", name).groups()) + (int(cluster.split(",")[2]),)
 """
+
+
+def test_products_stand_under_the_plan_they_take(run):                     # noqa: F811
+    run(PLAN_OF + f"""
+for (quant, kind), sizes in {PLANS}.items():
+    for want, size in sizes.items():
+        assert plan(quant, kind, *size) == want, (quant, kind, size, want, plan(quant, kind, *size))
+""")
+
+
+def test_no_model_takes_a_plan_that_is_not_tested(run):                    # noqa: F811
+    """The products of the table's models and of the designs' two sizes, at token counts over the whole range of a portion."""
+    designs = [(1536, 13440), (13440, 1536), (1536, 1536), (576, 1536), (6400, 1536), (1536, 6400), (8064, 1536), (64, 1536), (3584, 25600), (25600, 3584), (3584, 3584),
+               (12928, 3584), (3584, 12928), (1024, 3584), (16896, 3584)]
+    run(PLAN_OF + f"""
+tested = {PLANS}
+tokens = sorted(set(list(range(1, 300, 13)) + [int(1.11 ** i) for i in range(1, 87)] + [128, 129, 256, 257, 512, 513, 8192]))
+for n in tokens:
+    for m in binfmt.MODELS.values():
+        for quant in (0, 1, 2):
+            for kind, rows, cols in (("plain", (m["heads"] + 2 * m["kv"]) * m["hd"], m["dim"]), ("plain", m["dim"], m["heads"] * m["hd"]), ("swiglu", m["inter"], m["dim"]), ("plain", m["dim"], m["inter"])):
+                assert plan(quant, kind, n, rows, cols) in tested[quant, kind], (quant, kind, n, rows, cols)
+    for rows, cols in {designs}:
+        if 2 <= n <= 4096:
+            assert plan(3, "plain", n, rows, cols) in tested[3, "plain"], (n, rows, cols)
+""")
 
 
 def test_a_plan_on_any_number_of_sms(run):                                 # noqa: F811
