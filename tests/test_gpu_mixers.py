@@ -384,8 +384,8 @@ def test_long_decoding(models, act):
 
 
 @pytest.mark.parametrize("act", ACTS)
-def test_portions_longer_than_a_chunk(models, act):
-    """More tokens than go through the layers together; the first tokens after the border are one and several."""
+def test_long_portions(models, act):
+    """Portions of some 2000 tokens, and what follows them: one token and several."""
     d, cfg, wf, _, _ = models("small")
     toks = np.random.default_rng(4).integers(0, cfg["vocab"], 2100)
     want = M.forward(cfg, wf, toks)
@@ -400,17 +400,18 @@ def test_portions_longer_than_a_chunk(models, act):
     eng.close()
 
 
-def test_portions_beyond_4096_tokens(models):
+@pytest.mark.parametrize("act", ACTS)
+def test_portions_beyond_4096_tokens(models, act):
     """The border at which a portion is cut, one and several tokens behind it, and a workspace that grows on the way there."""
     d, cfg, wf, _, _ = models("small")
     toks = np.random.default_rng(5).integers(0, cfg["vocab"], 4140)
     want = M.forward(cfg, wf, toks)
-    eng = E.Engine.open(d, max_seq_len=4140)
-    check(eng.extend(toks[:300], 0, [299]), want[299][None], "bfloat16", 1.5)
+    eng = E.Engine.open(d, act=act, max_seq_len=4140)
+    check(eng.extend(toks[:300], 0, [299]), want[299][None], act, 1.5)
     for n in (4140, 4097):
         places = [p for p in (0, 63, 2048, 4094, 4095, 4096, 4097, 4103, 4139) if p < n]
-        check(eng.extend(toks[:n], 0, places), want[places], "bfloat16", 1.5)
-    check(eng.extend(toks[4097:4100], 4097, [0, 1, 2]), want[4097:4100], "bfloat16", 1.5)
+        check(eng.extend(toks[:n], 0, places), want[places], act, 1.5)
+    check(eng.extend(toks[4097:4100], 4097, [0, 1, 2]), want[4097:4100], act, 1.5)
     eng.close()
 
 

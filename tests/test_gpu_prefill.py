@@ -236,9 +236,9 @@ def test_prefill_vs_reference_build_token_by_token(built, tmpdir_big, model, qua
     assert agree == steps and worst <= 1.5e-2
 
 
-def test_prefill_longer_than_one_chunk_and_single_token(built, tmp_path):
-    """A prompt longer than the 2048-token chunk the engine works in (the second chunk attends to the first one's
-    rows), and the smallest call (one token at an odd position), against the token-by-token path."""
+def test_prefill_in_two_long_calls_and_single_token(built, tmp_path):
+    """A long prompt in two calls (the second one attends to the first one's rows), and the smallest call (one token at an odd position),
+    against the token-by-token path."""
     from cuqwen_b200 import engine as E
     cfg = dict(vocab=512, dim=256, inter=512, layers=2, heads=2, kv=1, hd=128, tied=True)
     path = tmp_path / "m.bin"
@@ -256,7 +256,8 @@ def test_prefill_longer_than_one_chunk_and_single_token(built, tmp_path):
     a, b = make(), make()
     for i in range(n + 1):
         a.step(int(toks[i]), i)
-    b.prefill(toks[:n], 0)
+    b.prefill(toks[:2048], 0)
+    b.prefill(toks[2048:n], 2048)
     b.prefill(toks[n:n + 1], n)
     shape = (cfg["layers"], cfg["kv"], max_seq, cfg["hd"])
     for which in ("KEY_CACHE", "VALUE_CACHE"):
@@ -264,7 +265,7 @@ def test_prefill_longer_than_one_chunk_and_single_token(built, tmp_path):
         cb = b.read(which).reshape(shape).astype(np.float64)[:, :, :n + 1]
         rms = np.sqrt(((ca - cb) ** 2).mean()) / np.sqrt((ca ** 2).mean())
         tail = np.sqrt(((ca[:, :, 2048:] - cb[:, :, 2048:]) ** 2).mean()) / np.sqrt((ca[:, :, 2048:] ** 2).mean())
-        print(f"{which}: rel rms {rms:.2e} (rows of the second chunk {tail:.2e})")
+        print(f"{which}: rel rms {rms:.2e} (rows of the second call {tail:.2e})")
         assert rms < 5e-3 and tail < 5e-3
     ta, tb = a.step(int(toks[n + 1]), n + 1), b.step(int(toks[n + 1]), n + 1)
     la, lb = a.read("LOGITS").astype(np.float64), b.read("LOGITS").astype(np.float64)
@@ -357,18 +358,33 @@ def test_prefill_attention_with_pairs_of_query_tiles(built, hd, T, pos0, nh, nkv
     test_prefill_attention_kernels(built, 0, hd, T, pos0, nh, nkv)
 
 
+@pytest.mark.parametrize("rows", ["all", "some"])
 @pytest.mark.parametrize("hd", [128, 64])
-def test_prefill_attention_moves_its_exponent(built, hd):
-    """Scores that grow from key tile to key tile by far more than 2^8, so that every tile rescales what has been summed."""
+@pytest.mark.parametrize("T,nh,nkv", [(300, 2, 1), (300, 228, 76)])
+def test_prefill_attention_moves_its_exponent(built, hd, rows, T, nh, nkv):
+    """Scores whose maximum grows from 128-key tile to 128-key tile by more than the kernel lets pass (2^8), so that every tile rescales what has
+    been summed: for every query, or for every third one (the rows of a warp then differ).  One query tile to a CTA and two."""
     rng = np.random.default_rng(hd)
-    T, nh, nkv, max_seq = 300, 2, 1, 640
-    q = np.abs(rng.standard_normal((T, nh * hd))).astype(np.float16)
+    max_seq, pos0 = 640, 330
+    q = np.abs(rng.standard_normal((T, nh, hd)))
+    if rows == "some":
+        q[np.arange(T) % 3 > 0] *= 0.01
+    q = q.reshape(T, nh * hd).astype(np.float16)
     Kc = rng.standard_normal((nkv, max_seq, hd)).astype(np.float16)
-    Kc += (np.arange(max_seq) // 100 * 0.5).astype(np.float16)[None, :, None]
+    Kc += (np.arange(max_seq) // 128 * (1.5 if hd == 128 else 2.6)).astype(np.float16)[None, :, None]
     Vc = rng.standard_normal((nkv, max_seq, hd)).astype(np.float16)
+    # the maxima that the kernel sees, in powers of two, tile by tile: those of the queries that are to move rise by more than 8 each time
+    kv = np.repeat(Kc, nh // nkv, axis=0).astype(np.float64)
+    x = np.einsum("thd,hkd->htk", q.reshape(T, nh, hd).astype(np.float64), kv) * (np.log2(np.e) / np.sqrt(hd))
+    x[:, np.arange(max_seq)[None, :] > pos0 + np.arange(T)[:, None]] = -np.inf
+    top = x.reshape(nh, T, max_seq // 128, 128).max(axis=3)
+    move = np.arange(T) % 3 == 0 if rows == "some" else np.ones(T, bool)
+    for t in range(T):
+        rise = np.diff(top[:, t, :(pos0 + t) // 128 + 1], axis=1)
+        assert (rise > 8.5).all() if move[t] else (rise < 7.5).all(), (t, rise.min(), rise.max())
     out = DevBuf(T * nh * hd * 2)
-    K.prefill_attention(0, dev(q), dev(Kc), dev(Vc), out, T, 330, nh, nkv, hd, max_seq)
+    K.prefill_attention(0, dev(q), dev(Kc), dev(Vc), out, T, pos0, nh, nkv, hd, max_seq)
     sync()
-    want = attn_oracle(q, Kc, Vc, 330, nh, nkv, hd)
+    want = attn_oracle(q, Kc, Vc, pos0, nh, nkv, hd)
     got = out.numpy(np.float16).reshape(T, nh * hd)
     assert close(got, want), report(got, want)

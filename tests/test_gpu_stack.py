@@ -314,8 +314,8 @@ def test_long_decoding_and_keys_that_left_every_window(models, act):
     assert not np.array_equal(out[0][180:196], out[1][180:196])
 
 
-def test_portions_longer_than_a_chunk(models):
-    """More tokens than go through the layers together, wanted places on both sides of the border; bfloat16."""
+def test_long_portions(models):
+    """Some 2000 tokens at once, wanted places at tile borders and anywhere; bfloat16."""
     d, cfg, wf, _, _ = models("small")
     n = 2100
     toks = np.random.default_rng(4).integers(0, cfg["vocab"], n)
@@ -330,16 +330,17 @@ def test_portions_longer_than_a_chunk(models):
     eng.close()
 
 
-def test_portions_beyond_4096_tokens(models):
+@pytest.mark.parametrize("act", ACTS)
+def test_portions_beyond_4096_tokens(models, act):
     """The border at which a portion is cut, and a workspace that grows on the way there."""
     d, cfg, wf, _, _ = models("small")
     n = 4160
     toks = np.random.default_rng(5).integers(0, cfg["vocab"], n)
-    eng = E.Engine.open(d, max_seq_len=n)
+    eng = E.Engine.open(d, act=act, max_seq_len=n)
     eng.extend(toks[:300], 0, [299])
     places = [4000, 4094, 4095, 4096, 4097, 4103, 4159]
     got = eng.extend(toks, 0, places)
-    check(got, np.concatenate([L.forward(cfg, wf, toks[p - 40:p + 1])[-1:] for p in places]), "bfloat16", 1.5)
+    check(got, np.concatenate([L.forward(cfg, wf, toks[p - 40:p + 1])[-1:] for p in places]), act, 1.5)
     eng.close()
 
 
