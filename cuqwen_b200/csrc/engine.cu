@@ -29,6 +29,7 @@
 #include "gemv_seg.cuh"
 #include "stack.h"
 #include "stack_host.h"
+#include "step_layers.h"
 #include "tp_plan.h"
 
 using namespace cq;
@@ -247,6 +248,8 @@ extern "C" void cuqwen_destroy(cuqwen_engine* e) {
     for (void* b : bufs) if (b) cudaFree(b);
     if (e->h_ctl) cudaFreeHost(e->h_ctl);
     if (e->hio) cudaFreeHost(e->hio);
+    if (e->layers_words) cudaFree(e->layers_words);
+    delete e->layers_args;
     if (e->h_out) cudaFreeHost(e->h_out);
     stack_destroy(e);
     if (e->ev0) cudaEventDestroy(e->ev0);
@@ -377,6 +380,49 @@ static int walk_file(cuqwen_engine* e, Cursor cur, Arena& ar, int lm_fmt) {
     return CUQWEN_OK;
 }
 
+// Prepares the step whose layers are one kernel (step_layers.h), where this engine can take it; an engine that cannot keeps the launch-by-launch step: tensor
+// parallelism and the 8-bit cache, whose exchanges and rows the kernel does not know; a timeline or a switched-off hand-over, which speak of the separate launches; the accurate
+// rotation, the mode in which kernels are compared with the oracle one by one; shapes beyond the plan; a device without cooperative launches.
+static int prepare_layers(cuqwen_engine* e) {
+    const cuqwen_params& p = e->p;
+    int coop = 0;
+    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, p.device));
+    if (!coop || e->tp > 1 || e->kv8 || (p.flags & (CUQWEN_FLAG_STEP_TRACE | CUQWEN_FLAG_NO_HANDOVER | CUQWEN_FLAG_ACCURATE_ROPE))) return CUQWEN_OK;
+    const StepShape sh{p.quant, p.dim, p.intermediate_size, p.n_heads, p.n_kv_heads, p.head_dim, p.n_layers, p.max_seq_len, e->nsplit, e->sms};
+    StepArgs a; memset(&a, 0, sizeof a);
+    StepCore& c = a.c;
+    size_t words[7], total = 0;
+    if (!step_layers_plan(sh, c, words)) return CUQWEN_OK;
+    // the kernel finds a layer's tensors at one distance from the layer before: so the loader lays them out
+    auto tensors = [&](const Layer& L) {
+        return std::vector<const void*>{L.in_norm, L.q.w, L.q.s, L.bq, L.k.w, L.k.s, L.bk, L.v.w, L.v.s, L.bv, L.o.w, L.o.s, L.post_norm, L.gate.w, L.gate.s, L.up.w, L.up.s, L.down.w, L.down.s};
+    };
+    const std::vector<const void*> t0 = tensors(e->layers[0]);
+    c.layer_stride = p.n_layers > 1 ? (const char*)e->layers[1].in_norm - (const char*)t0[0] : 256;
+    for (int l = 1; l < p.n_layers; ++l) {
+        const std::vector<const void*> t = tensors(e->layers[l]);
+        for (size_t i = 0; i < t.size(); ++i) if (t0[i] && (const char*)t[i] != (const char*)t0[i] + c.layer_stride * l) return CUQWEN_OK;
+    }
+    const Layer& L = e->layers[0];
+    const void* const w[SM_COUNT] = {L.q.w, L.k.w, L.v.w, L.o.w, L.gate.w, L.up.w, L.down.w};
+    if (step_layers_maps(sh, a, w, e->kc, e->vc)) return CUQWEN_OK;
+    const Mat* const m[SM_COUNT] = {&L.q, &L.k, &L.v, &L.o, &L.gate, &L.up, &L.down};
+    for (int i = 0; i < SM_COUNT; ++i) c.scale[i] = m[i]->s;
+    c.bias[0] = L.bq; c.bias[1] = L.bk; c.bias[2] = L.bv; c.norm[0] = L.in_norm; c.norm[1] = L.post_norm;
+    c.x = e->x; c.q = e->q; c.k = e->k; c.v = e->v; c.att = e->att; c.gate = e->gate; c.kc = e->kc; c.vc = e->vc;
+    c.d_pos = &e->ctl->pos; c.err = reinterpret_cast<unsigned*>(&e->ctl->pad[0]);
+    c.eps = __half2float(__float2half(p.norm_eps)); c.scale_log2 = (1.0f / sqrtf((float)p.head_dim)) * 1.4426950408889634f; c.theta = p.rope_theta;
+    for (size_t& n : words) { n = align_up(n, 16); total += n; }
+    if (cudaMalloc((void**)&e->layers_words, total * 8 + 128) != cudaSuccess) { cudaGetLastError(); e->layers_words = nullptr; return CUQWEN_OK; }
+    CK(cudaMemsetAsync(e->layers_words, 0, total * 8 + 128, e->stream));          // a word's number is never 0
+    uint2** const at[7] = {&c.w_x1, &c.w_x2, &c.w_qkv, &c.w_part, &c.w_ml, &c.w_att, &c.w_h};
+    uint2* b = e->layers_words;
+    for (int i = 0; i < 7; ++i) { *at[i] = b; b += words[i]; }
+    e->epoch = reinterpret_cast<unsigned*>(b); c.epoch = e->epoch;
+    e->layers_args = new StepArgs(a);
+    return CUQWEN_OK;
+}
+
 extern "C" int cuqwen_load(cuqwen_engine* e, const char* path) {
     if (!e || !path) return fail(CUQWEN_ERR_ARG, "null argument");
     if (e->stack) return fail(CUQWEN_ERR_STATE, "cuqwen_open has loaded this engine's weights");
@@ -413,6 +459,7 @@ extern "C" int cuqwen_load(cuqwen_engine* e, const char* path) {
         CK(cudaMalloc((void**)&e->step_trace, e->step_trace_bytes));
         CK(cudaMemsetAsync(e->step_trace, 0, e->step_trace_bytes, e->stream));
     }
+    if (int r2 = prepare_layers(e)) return r2;
     e->loaded = true;
     return CUQWEN_OK;
 }
@@ -579,10 +626,15 @@ static int record_step(cuqwen_engine* e, cudaStream_t s, bool pdl) {
         e->launches = n;
         return CUQWEN_OK;
     }
-    LK(launch_embed_step(e->embed, e->ctl, e->x, p.dim, cfg_plain));
+    const bool one_kernel = e->layers_args && !e->prof;              // a profile times the separate launches
+    LK(launch_embed_step(e->embed, e->ctl, e->x, p.dim, cfg_plain, e->epoch));
     {
         std::vector<HostPhase> hp;
         describe_step(e, hp, e->nsplit);
+        if (one_kernel) {
+            LK(launch_step_layers(p.quant, *e->layers_args, cfg));
+            hp.erase(hp.begin(), hp.end() - 1);                      // the head is left
+        }
         for (HostPhase& h : hp) {
             unsigned long long* tr = e->step_trace && (size_t)(n + 2) * kTraceWords * 8 <= e->step_trace_bytes ? e->step_trace + (size_t)n * kTraceWords : nullptr;
             if (h.ph.kind == PH_ATTN) { h.ph.at.trace = tr; LK(launch_attn(p.head_dim, h.ph.at, cfg)); ++n; continue; }      // two launches: partials, fold

@@ -16,6 +16,7 @@
 namespace cq {
 
 struct Stack;
+struct StepArgs;
 
 struct Mat { uint8_t* w = nullptr; __half* s = nullptr; int rows = 0, cols = 0; };
 struct Layer {
@@ -54,6 +55,8 @@ struct cuqwen_engine {
     // peer exchange (tensor parallel without collective calls): one receive block per rank, mapped into every peer
     unsigned char* tp_rx = nullptr; size_t tp_rx_bytes = 0; unsigned char* peer_rx[8] = {}; bool tp_peer = false;
     __half* x2 = nullptr; bool tp_sum_separate = false;
+    // all layers of a step as one kernel (step_layers.h): its argument block, exchange words and step number; null: the step is launched kernel by kernel
+    cq::StepArgs* layers_args = nullptr; uint2* layers_words = nullptr; unsigned* epoch = nullptr;
     unsigned char* gate_xd = nullptr; int* gate_corr = nullptr; float* gate_xscale = nullptr;    // SwiGLU output in staged form (see GemvArgs::xd_out)
     unsigned char* att_xd = nullptr; int* att_corr = nullptr; float* att_xscale = nullptr;       // attention output in staged form (see AttnArgs::xd_out)
     // batched prefill workspace (cuqwen_prefill), for pf_rows tokens, grown when a longer portion comes

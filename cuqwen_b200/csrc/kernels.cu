@@ -7,6 +7,7 @@
 #include "gemv_stage.cuh"
 #include "launch.h"
 #include "rng.cuh"
+#include "tensor_map.h"
 
 #include <cstdio>
 #include <cstdlib>
@@ -40,7 +41,9 @@ int launch_embed(const __half* table, const int* d_token, __half* out, int dim, 
 // The same as the first launch of a decode step.  One CTA: thread 0 first takes over what the host left in the mailbox
 // (one 16-byte read of mapped host memory), the others wait for it, and only then are the dependent launches released -
 // a later kernel may read ctl->pos before its own dependency wait.
-__global__ void embed_step_kernel(const __half* __restrict__ table, StepCtl* ctl, __half* __restrict__ out, int dim) {
+// epoch (may be null): counts the steps that were begun, whatever became of them; a step's exchange words carry numbers that derive from it.
+__global__ void embed_step_kernel(const __half* __restrict__ table, StepCtl* ctl, __half* __restrict__ out, int dim, unsigned* epoch) {
+    if (threadIdx.x == 32 && epoch) *epoch += 1u;
     if (threadIdx.x == 0 && ctl->hio && !ctl->auto_advance) {
         int sq, tk, ps, hl;
         asm volatile("ld.volatile.global.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(sq), "=r"(tk), "=r"(ps), "=r"(hl) : "l"(ctl->hio) : "memory");
@@ -53,8 +56,8 @@ __global__ void embed_step_kernel(const __half* __restrict__ table, StepCtl* ctl
     uint4* dst = reinterpret_cast<uint4*>(out);
     for (int i = threadIdx.x; i < dim / 8; i += blockDim.x) dst[i] = src[i];
 }
-int launch_embed_step(const __half* table, StepCtl* ctl, __half* out, int dim, const LaunchCfg& cfg) {
-    return launch_k(embed_step_kernel, dim3(1), dim3(256), 0, cfg, table, ctl, out, dim);
+int launch_embed_step(const __half* table, StepCtl* ctl, __half* out, int dim, const LaunchCfg& cfg, unsigned* epoch) {
+    return launch_k(embed_step_kernel, dim3(1), dim3(256), 0, cfg, table, ctl, out, dim, epoch);
 }
 
 // ---- stand-alone RMSNorm (reference src/kernels.cu:689-751) ----------------
@@ -477,6 +480,27 @@ static int encode_weight_map(CUtensorMap* m, const void* w, size_t row_bytes, si
     const cuuint32_t box[3] = {kChunkBytes, (cuuint32_t)box_rows, (cuuint32_t)(piece_bytes / kChunkBytes)}, estr[3] = {1, 1, 1};
     CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+}
+
+int encode_layer_map(CUtensorMap* m, const void* w, size_t row_bytes, size_t rows, int layers, size_t layer_stride, int piece_bytes, int box_rows) {
+    EncodeTiledFn fn = encode_tiled();
+    if (!fn) return (int)cudaErrorNotSupported;
+    if (row_bytes % kChunkBytes || piece_bytes % kChunkBytes || layer_stride % 16) return (int)cudaErrorInvalidValue;
+    const cuuint64_t dims[4] = {kChunkBytes, rows, row_bytes / kChunkBytes, (cuuint64_t)layers}, strides[3] = {row_bytes, kChunkBytes, layer_stride};
+    const cuuint32_t box[4] = {kChunkBytes, (cuuint32_t)box_rows, (cuuint32_t)(piece_bytes / kChunkBytes), 1}, estr[4] = {1, 1, 1, 1};
+    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+}
+
+int encode_cache_map(CUtensorMap* m, const void* cache, size_t rows, int hd, int keys) {
+    EncodeTiledFn fn = encode_tiled();
+    if (!fn) return (int)cudaErrorNotSupported;
+    const cuuint64_t dims[3] = {64, rows, (cuuint64_t)hd / 64}, strides[2] = {(cuuint64_t)hd * 2, 128};
+    const cuuint32_t box[3] = {64, (cuuint32_t)keys, (cuuint32_t)hd / 64}, estr[3] = {1, 1, 1};
+    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(cache), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 

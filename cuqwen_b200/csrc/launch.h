@@ -59,7 +59,7 @@ size_t attn_scratch_counters(int n_kv, int nsplit);   // u32 tickets
 
 int launch_embed(const __half* table, const int* d_token, __half* out, int dim, const LaunchCfg& cfg);
 // First launch of a decode step: takes over a new mailbox message (unless the step feeds itself), then copies the token's row.
-int launch_embed_step(const __half* table, StepCtl* ctl, __half* out, int dim, const LaunchCfg& cfg);
+int launch_embed_step(const __half* table, StepCtl* ctl, __half* out, int dim, const LaunchCfg& cfg, unsigned* epoch = nullptr);
 int launch_rmsnorm(const __half* x, const __half* w, __half* out, int dim, float eps, const LaunchCfg& cfg);
 int launch_rope(__half* q, __half* k, int n_heads, int n_kv, int hd, const int* d_pos, float theta, int fast, const LaunchCfg& cfg);
 int launch_kv_store(const __half* k, const __half* v, __half* kc, __half* vc, const int* d_pos, int n_kv, int max_seq, int hd, const LaunchCfg& cfg);

@@ -1,0 +1,8 @@
+// The step's layers for one weight format.
+#include "step_layers.cuh"
+
+namespace cq {
+
+int launch_step_layers_i8(const StepArgs& a, const LaunchCfg& cfg) { return launch_step_layers_q<Q_I8>(a, cfg); }
+
+}  // namespace cq

@@ -1,0 +1,109 @@
+"""A step whose layers are one kernel, against the oracle and against the launch-by-launch step of the same model, at the sizes where its work split, its ring
+and its key ranges have their edges."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from cuqwen_b200 import _abi, binfmt
+from cuqwen_b200 import engine as E
+from oracle import oracle_py as O
+from tests.gpu_util import close, report
+
+pytestmark = pytest.mark.gpu
+
+MODELS = {
+    # one K-part to sixteen, blocks of 8 and 40 rows, seven query heads a KV head
+    "0.5b": dict(vocab=1024, dim=896, inter=4864, layers=3, heads=14, kv=2, hd=64, tied=True),
+    # two q/k/v blocks in a CTA (224 on 148 SMs), the attention wider than the model, 18 key ranges a head, five query heads
+    "wide attention": dict(vocab=1024, dim=256, inter=640, layers=3, heads=40, kv=8, hd=128, tied=False),
+    # SwiGLU output as digits; one KV head
+    "wide mlp": dict(vocab=1024, dim=256, inter=18944, layers=3, heads=8, kv=1, hd=64, tied=True),
+    # the smallest: most CTAs have no work in most phases
+    "one": dict(vocab=512, dim=128, inter=128, layers=1, heads=1, kv=1, hd=128, tied=True),
+    # three tiles of rows a block, blocks that end beyond the matrix
+    "ragged": dict(vocab=512, dim=5120, inter=1408, layers=1, heads=2, kv=2, hd=128, tied=True),
+}
+MAX_SEQ = 1600
+
+
+def make(cfg, quant, path, flags=0, splits=0):
+    p = E.custom_params(cfg["vocab"], cfg["dim"], cfg["inter"], cfg["layers"], cfg["heads"], cfg["kv"], cfg["hd"], quant, max_seq_len=MAX_SEQ)
+    p.flags, p.attn_splits = flags, splits
+    e = E.Engine(p)
+    e.load(str(path))
+    return e
+
+
+def poison(eng, cfg, first):
+    """NaN in every cached row from `first` on."""
+    rows = np.full((MAX_SEQ - first) * cfg["hd"], np.nan, np.float16)
+    for which in ("KEY_CACHE", "VALUE_CACHE"):
+        base = eng.ptr(which)[0]
+        for lh in range(cfg["layers"] * cfg["kv"]):
+            assert _abi.lib().cuqwen_dev_upload(0, base + (lh * MAX_SEQ + first) * cfg["hd"] * 2, rows.ctypes.data_as(ctypes.c_void_p), rows.nbytes) == 0
+
+
+@pytest.mark.parametrize("name", list(MODELS))
+@pytest.mark.parametrize("quant", [0, 1, 2])
+def test_against_the_separate_launches(built, tmp_path, name, quant):
+    """Same weights, same caches, contexts around the edges of a stage (32 or 64 keys), of a key range and of sixteen stages (one key range a head).  Both steps round the same vectors
+    to fp16, from sums in different orders (and the kernel does not round normalised activations of quantised weights): six vectors a layer, each off by at most half a unit in the last
+    place, 2^-11 relative, of a value of its own size; over three layers the 2-norms differ by sqrt(18) / sqrt(3) x 2^-11 = 1.2e-3, of which four times is asked."""
+    cfg = MODELS[name]
+    path = tmp_path / "m.bin"
+    binfmt.write_model(path, cfg, quant, binfmt.random_tensors(cfg, 5))
+    for splits, contexts in ((0, (0, 1, 31, 32, 33, 63, 64, 65, 127, 500, 1599)), (1, (40, 513, 1200))):
+        a, b = make(cfg, quant, path, 0, splits), make(cfg, quant, path, E.FLAG_NO_HANDOVER, splits)
+        for ctx in contexts:
+            for e in (a, b):
+                e.kv_fill_normal(ctx, 7)
+                poison(e, cfg, ctx)
+                e.step(3 + ctx % 100, ctx)
+            assert a.step_launches == 5 and b.step_launches == 1 + 6 * cfg["layers"] + 3
+            la, lb = a.read("LOGITS").astype(np.float64), b.read("LOGITS").astype(np.float64)
+            assert np.linalg.norm(la - lb) <= 5e-3 * np.linalg.norm(lb), (ctx, np.linalg.norm(la - lb) / np.linalg.norm(lb))
+            for which in ("X", "Q", "K", "V", "ATT", "GATE"):          # what a program may read after a step
+                va, vb = a.read(which).astype(np.float64), b.read(which).astype(np.float64)
+                assert np.linalg.norm(va - vb) <= 5e-3 * np.linalg.norm(vb), (ctx, which)
+            ka, kb = (e.read("KEY_CACHE").reshape(cfg["layers"], cfg["kv"], MAX_SEQ, cfg["hd"]) for e in (a, b))
+            assert np.isfinite(ka[:, :, :ctx + 1]).all() and np.isnan(ka[:, :, ctx + 1:]).all() and close(ka[:, :, ctx], kb[:, :, ctx])
+        a.close()
+        b.close()
+
+
+@pytest.mark.parametrize("name", ["0.5b", "wide attention"])
+@pytest.mark.parametrize("quant", [0, 1, 2])
+def test_against_the_oracle(built, tmp_path, name, quant):
+    cfg = MODELS[name]
+    path = tmp_path / "m.bin"
+    binfmt.write_model(path, cfg, quant, binfmt.random_tensors(cfg, 6))
+    eng, orc = make(cfg, quant, path), O.OracleModel(str(path), MAX_SEQ)
+    for pos, tok in enumerate(np.random.default_rng(8).integers(0, cfg["vocab"], 36)):
+        eng.step(int(tok), pos)
+        orc.step(int(tok), pos)
+        assert close(eng.read("LOGITS"), orc.logits), (pos, report(eng.read("LOGITS"), orc.logits))
+    assert eng.step_launches == 5
+    eng.close()
+    orc.close()
+
+
+def test_steps_of_two_engines_do_not_mix(built, tmp_path):
+    """Their exchange words are their own, and a step's numbers go on when the control block is written anew (decode_n, a profile, which runs the separate launches)."""
+    cfg = MODELS["0.5b"]
+    path = tmp_path / "m.bin"
+    binfmt.write_model(path, cfg, 2, binfmt.random_tensors(cfg, 9))
+    a, b, c = (make(cfg, 2, path) for _ in range(3))
+    want = [a.step(5, 0)]
+    for i in range(1, 24):
+        want.append(a.step(want[-1], i))
+    got = b.decode_n(5, 0, 8).tolist()
+    b.profile_step(got[-1], 8)
+    other = c.step(9, 0)
+    for i in range(8, 16):
+        got.append(b.step(got[-1], i))
+        other = c.step(other, i - 7)
+    got += b.decode_n(got[-1], 16, 8).tolist()
+    assert got == want
+    for e in (a, b, c):
+        e.close()

@@ -1,0 +1,38 @@
+"""Which engines run a step's layers as one kernel, and which launch by launch, on the CPU over tests/cudart_stub.cpp."""
+import pytest
+
+from cuqwen_b200 import binfmt
+from test_host_memory import run                                           # noqa: F401  (fixture)
+
+PLAIN = dict(vocab=512, dim=256, inter=512, layers=2, heads=4, kv=2, hd=64, tied=True)
+
+
+def kernels_of_a_step(run, tmp_path, cfg, quant, flags="0", splits=0, sms=148):      # noqa: F811
+    path = tmp_path / "m.bin"
+    binfmt.write_model(path, cfg, quant, binfmt.random_tensors(cfg, 3))
+    return run(f"""
+stub.stub_sms({sms})
+p = E.custom_params({cfg['vocab']}, {cfg['dim']}, {cfg['inter']}, {cfg['layers']}, {cfg['heads']}, {cfg['kv']}, {cfg['hd']}, {quant}, max_seq_len=256)
+p.flags = E.FLAG_NO_GRAPH | {flags}
+p.attn_splits = {splits}
+eng = E.Engine(p)
+eng.load(sys.argv[1])
+stub.stub_launches()
+eng.step(1, 0)
+print(stub.stub_launches().decode())
+assert eng.step_launches == (5 if "{flags}" == "0" and {splits} * {cfg['kv']} <= {sms} and {cfg['heads']} <= {sms} else 1 + 6 * {cfg['layers']} + 3)
+""", path)
+
+
+@pytest.mark.parametrize("quant", [0, 1, 2])
+@pytest.mark.parametrize("hd", [64, 128])
+def test_the_layers_of_a_step_are_one_launch(run, tmp_path, quant, hd):     # noqa: F811
+    out = kernels_of_a_step(run, tmp_path, dict(PLAIN, hd=hd), quant).split("\n")
+    names = [n for n in out if n]
+    assert len(names) == 5 and "step_layers_kernel" in names[1] and " 148,1,1 " in names[1] and "gemv_kernel" in names[2]
+
+
+@pytest.mark.parametrize("flags,splits,sms", [("E.FLAG_ACCURATE_ROPE", 0, 148), ("E.FLAG_NO_HANDOVER", 0, 148), ("E.FLAG_STEP_TRACE", 0, 148), ("E.FLAG_KV_INT8", 0, 148),
+                                              ("0", 75, 148), ("0", 0, 3)])
+def test_what_the_kernel_does_not_know_stays_launch_by_launch(run, tmp_path, flags, splits, sms):      # noqa: F811
+    assert "step_layers_kernel" not in kernels_of_a_step(run, tmp_path, PLAIN, 2, flags, splits, sms)
