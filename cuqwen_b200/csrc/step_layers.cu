@@ -47,6 +47,12 @@ bool step_layers_plan(const StepShape& s, StepCore& a, size_t (&words)[7]) {
     if (a.staged_h) rows_mlp = 128;
     // a slot: 16 KB (keys and values of 32 or 64 tokens), or what one unit of the widest phase needs
     a.slot_bytes = 2 * rows_mlp * gb > 16 * 1024 ? (2 * rows_mlp * gb + 1023) / 1024 * 1024 : 16 * 1024;
+    // ... or one unit of each K-part, where that is little more (0.5B fp16: gate/up blocks of 34 rows, 17 KB)
+    auto widen = [&](int rows, int mt, int K) {
+        const int kp = kWarps / (mt * ((rows + 15) / 16)), U = K / unit_cols(s.quant), want = mt * rows * gb * (kp < U ? kp : U);
+        if (want > a.slot_bytes && want <= 20 * 1024) a.slot_bytes = (want + 1023) / 1024 * 1024;
+    };
+    widen(16, 2, s.dim); widen(rows_out, 1, qd); widen(rows_mlp, 2, s.dim); widen(rows_out, 1, s.inter);
     auto phase = [&](int i, int K, int rows, int all, int nblk, int mt) {
         StepGemv& g = a.g[i];
         g.K = K; g.ngrp = K / kGroup; g.brows = rows; g.nblk = nblk; g.nb = (nblk + s.sms - 1) / s.sms; g.mt = mt; g.rt = (rows + 15) / 16; g.nt = mt * g.rt; g.kp = kWarps / g.nt; g.rows = all;
@@ -73,8 +79,8 @@ bool step_layers_plan(const StepShape& s, StepCore& a, size_t (&words)[7]) {
     auto take = [&](int bytes, int align) { o = (o + align - 1) / align * align; const int at = o; o += bytes; return at; };
     a.off_x = take(area, 128);
     a.off_corr = take(K / kGroup * 8, 16); a.off_job = take(SP_COUNT * kWarps * 16, 16);
-    a.off_zero = take(160, 16); a.off_red = take(2 * kWarps * 17 * 4, 16); a.off_rms = take(kWarps * 4, 16);
-    a.off_q = take(kMaxGroup * s.hd * 2, 16); a.off_cur = take(s.hd == 128 ? 32 * 128 + 256 : 256, 128); a.off_hbuf = take(256 + 264 + 8, 16);
+    a.off_zero = take(256, 16); a.off_red = take(2 * kWarps * 17 * 4, 16); a.off_rms = take(kWarps * 4, 16);
+    a.off_q = take(kMaxGroup * (s.hd * 2 + 64), 16); a.off_cur = take(s.hd == 128 ? 32 * 128 + 256 : 256, 128); a.off_hbuf = take(256 + 264 + 8, 16);
     a.off_res = take(a.g[SP_O].nb * rows_out * 2, 16); a.off_rope = take(a.g[SP_QKV].nb * 16 * 8, 16); a.off_range = take(64, 16);
     for (int i = 0; i < SP_COUNT; ++i) a.g[i].off_scale = take(a.g[i].nb * a.g[i].scale_bytes, 128);
     a.off_ring = take(0, 1024);            // (the swizzle's pattern)

@@ -71,22 +71,25 @@ __device__ __forceinline__ void step_wait(StepRing& R, uint32_t bar, uint32_t pa
     while (!mbar_try_wait(bar, parity))
         if (cycles32() - t0 > 2000000000u) { R.failed = code; return; }
 }
-// Polls N pairs of words, `stride` words apart, until all carry `seq`; bounded by 2^20 tries of an L2 round trip each (some 0.3 s: less than the ring's limit, which therefore does
+// Polls N pairs of words, `stride` words apart, and (EXTRA) the pair at q, until all carry `seq`; bounded by 2^20 tries of an L2 round trip each (some 0.3 s: less than the ring's limit, which therefore does
 // not expire with it); after that the thread polls no more in this step.  The ring goes on, so that no copy is under way when the CTA ends.
-template <int N>
-__device__ __forceinline__ void poll_words(StepRing& R, const uint2* p, int stride, uint32_t seq, uint32_t (&v)[2 * N]) {
+template <int N, int EXTRA = 0>
+__device__ __forceinline__ void poll_words(StepRing& R, const uint2* p, int stride, const uint2* q, uint32_t seq, uint32_t (&v)[2 * (N + EXTRA)]) {
 #pragma unroll 1
     for (int tries = 1 << 20;; --tries) {
         uint32_t bad = 0;
-        unsigned long long a[N], b[N];
+        unsigned long long a[N + EXTRA], b[N + EXTRA];
 #pragma unroll
         for (int i = 0; i < N; ++i) ld_word2(p + i * stride, a[i], b[i]);
+        if (EXTRA) ld_word2(q, a[N + EXTRA - 1], b[N + EXTRA - 1]);
 #pragma unroll
-        for (int i = 0; i < N; ++i) { v[2 * i] = (uint32_t)a[i]; v[2 * i + 1] = (uint32_t)b[i]; bad |= ((uint32_t)(a[i] >> 32) ^ seq) | ((uint32_t)(b[i] >> 32) ^ seq); }
+        for (int i = 0; i < N + EXTRA; ++i) { v[2 * i] = (uint32_t)a[i]; v[2 * i + 1] = (uint32_t)b[i]; bad |= ((uint32_t)(a[i] >> 32) ^ seq) | ((uint32_t)(b[i] >> 32) ^ seq); }
         if (bad == 0 || R.poll_failed) return;
         if (tries == 0) R.poll_failed = 11u;
     }
 }
+template <int N>
+__device__ __forceinline__ void poll_words(StepRing& R, const uint2* p, int stride, uint32_t seq, uint32_t (&v)[2 * N]) { poll_words<N, 0>(R, p, stride, nullptr, seq, v); }
 
 // Shared memory of a CTA; the argument block lies at its start, where the consumers' phases read it: read from the parameters, the compiler carries the phases' constants
 // through all layers, in registers that sixteen warps (112 a thread) do not have.
@@ -119,6 +122,10 @@ struct StepLayers {
 
     // ---- producer -----------------------------------------------------------
     static constexpr int kRowB = HD * 2, kKeys = HD == 128 ? 32 : 64, kHalf = kKeys * kRowB, kPer = kKeys / 32;      // keys of a stage, warps that share one
+    static constexpr int kRowQ = kRowB + 64;      // a row of q in shared memory: two of them in different banks
+    // Contexts of up to so many keys are one range a KV head, eight or nine warps' work, and its CTA writes the attention's output itself: the merge of partials, a hand-over and some 2000
+    // cycles, falls away (us a step, 0.5B int4 at 120 keys 432 -> 413, at 250 434 -> 425; at 500 nothing: one SM streams all keys of a head).
+    static constexpr int kDirect = 256;
     // A free slot for the next stage, whose barrier then expects `tx` bytes.  One thread issues all copies of an SM, some 40 instructions a stage
     // (slots of one size: with stages packed behind one another it took 90, and was what the large matrices waited for).
     static __device__ __forceinline__ uint32_t claim(StepRing& R, uint32_t full, uint32_t slots, uint32_t tx) {
@@ -179,7 +186,7 @@ struct StepLayers {
         const int cta = blockIdx.x;
         r.pos = *a.d_pos;
         r.kvh = cta / a.nsplit; r.split = cta - r.kvh * a.nsplit;
-        const int len = r.pos + 1, chunk = attn_chunk(len, a.nsplit);
+        const int len = r.pos + 1, chunk = len <= kDirect ? kDirect : attn_chunk(len, a.nsplit);
         r.t0 = r.split * chunk;
         const int t1 = min(r.t0 + chunk, len);
         r.any = r.kvh < a.n_kv && r.t0 < len;
@@ -188,7 +195,7 @@ struct StepLayers {
         r.nstage = r.any ? (r.t1c - r.t0 + kKeys - 1) / kKeys : 0;
         r.nne = (len + chunk - 1) / chunk;            // key ranges that are not empty
         const int per_head = gridDim.x / a.n_heads;
-        r.fold_head = cta % per_head == 0 && cta / per_head < a.n_heads ? cta / per_head : -1;
+        r.fold_head = r.nne > 1 && cta % per_head == 0 && cta / per_head < a.n_heads ? cta / per_head : -1;
         for (int i = 0; i < SP_COUNT; ++i) r.nb[i] = cta < a.g[i].nblk ? (a.g[i].nblk - cta + (int)gridDim.x - 1) / (int)gridDim.x : 0;
         return r;
     }
@@ -526,7 +533,7 @@ struct StepLayers {
     // chunk j at place j ^ (r & 7).  Lane g of a fragment takes key (and chunk of V) perm(g) instead of g, so that the eight lanes of a quarter-warp, two g by four t, read eight
     // different places; of rows as they are cached, 256 bytes apart, 2 lanes of K and 4 of V met in a bank.  n: keys that exist.
     static __device__ __forceinline__ int perm(int g) { return g >> 1 | (g & 1) << 2; }
-    static __device__ __forceinline__ void tile(AttnState<HD>& st, const uint32_t (&qa)[HD / 32][4], uint32_t sK, uint32_t sV, int n, float scale, int g, int t) {
+    static __device__ __forceinline__ void tile(AttnState<HD>& st, uint32_t sQ, uint32_t sK, uint32_t sV, int n, float scale, int g, int t) {
         constexpr int NCH = HD / 32, NC = HD / 64, NMT = HD / 16, COLS = kKeys * 128;
         const uint32_t k0 = sK + perm(g) * 128 + ((t ^ perm(g)) << 4), k1 = sK + perm(g) * 128 + ((4 + t ^ perm(g)) << 4);
         const uint32_t v0 = sV + t * 128 + ((t ^ perm(g)) << 4), v1 = sV + (t + 4) * 128 + ((t + 4 ^ perm(g)) << 4);
@@ -535,13 +542,14 @@ struct StepLayers {
         for (int b = 0; b < 4; ++b) sc[b][0] = sc[b][1] = sc[b][2] = sc[b][3] = 0.f;
 #pragma unroll
         for (int i = 0; i < NCH; ++i) {
+            const uint4 qf = lds128(sQ + i * 64);
             uint4 kf[4];
 #pragma unroll
             for (int b = 0; b < 4; ++b) kf[b] = lds128((i & 1 ? k1 : k0) + (i >> 1) * COLS + b * 1024);
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
-                mma16816(sc[b], qa[i][0], 0u, qa[i][1], 0u, kf[b].x, kf[b].y);
-                mma16816(sc[b], qa[i][2], 0u, qa[i][3], 0u, kf[b].z, kf[b].w);
+                mma16816(sc[b], qf.x, 0u, qf.y, 0u, kf[b].x, kf[b].y);
+                mma16816(sc[b], qf.z, 0u, qf.w, 0u, kf[b].z, kf[b].w);
             }
         }
         float mx = -INFINITY;
@@ -595,15 +603,15 @@ struct StepLayers {
     }
 
     // Attention over this CTA's key range for the query heads of its KV head.
-    static __device__ __forceinline__ void attend(uint32_t seq, StepRing& R) {
-        constexpr int NCH = HD / 32, NMT = HD / 16;
+    static __device__ __forceinline__ void attend(uint32_t seq, bool last, StepRing& R) {
+        constexpr int NMT = HD / 16;
         const StepCore& a = core();
         unsigned char* sm = step_smem;
         const uint32_t sm0 = smem_u32(step_smem);
         const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-        const Range r = range(a);
+        const Range& r = range(a);
         const int grp = a.grp;
-        unsigned char* qs = sm + a.off_q;                            // [kMaxGroup][HD]; the step's own key and value as row 0 of a stage of their own (V 128 bytes behind K)
+        unsigned char* qs = sm + a.off_q;                            // rows of q; the step's own key and value as row 0 of a stage of their own (V 128 bytes behind K)
         {
             const int nq = grp * HD / 4, j = tid - kStepConsumers / 2;           // pairs of words: of q by the first half of the threads, of k and v by the next ones
             const bool isq = tid < nq, isk = j < HD / 4;
@@ -613,34 +621,28 @@ struct StepLayers {
                 uint32_t v[2];
                 poll_words<1>(R, a.w_qkv + h0 * (HD / 2) + 2 * u, 0, seq, v);
                 const int hl = 2 * u / (HD / 2), d = 2 * u - hl * (HD / 2);
-                unsigned char* o = isq ? qs + (hl * HD + d) * 2 : sm + a.off_cur + (isk ? 0 : 128) + d * 2;
+                unsigned char* o = isq ? qs + hl * kRowQ + d * 2 : sm + a.off_cur + (isk ? 0 : 128) + d * 2;
                 *reinterpret_cast<uint32_t*>(o) = prmt(v[0], v[1], 0x5410);
                 *reinterpret_cast<uint32_t*>(o + (isq || HD == 64 ? HD : kKeys * 128)) = prmt(v[0], v[1], 0x7632);
             }
         }
         consumer_sync(kStepConsumers);
-        uint32_t qa[NCH][4];
-#pragma unroll
-        for (int i = 0; i < NCH; ++i) {
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (g < grp) v = lds128(sm0 + a.off_q + g * kRowB + (i * 4 + t) * 16);
-            qa[i][0] = v.x; qa[i][1] = v.y; qa[i][2] = v.z; qa[i][3] = v.w;
-        }
+        const uint32_t sQ = g < grp ? sm0 + a.off_q + g * kRowQ + t * 16 : sm0 + a.off_zero;        // (heads that do not exist: zeros)
         AttnState<HD> st;
         st.reset();
         // A warp waits for its own stages only and lets the others go at once.  That is safe with 32 barriers and at most 16 slots: it is at most 15 stages past one that it saw full, before
         // which all but the last `slots` stages had been let go by all warps, so no warp is still to arrive at the barrier's use before.
-        const int ns = r.nstage + r.own;                             // the step's own key and value are one more stage, of one key, outside the ring
+        const int nstage = r.nstage, keys = r.t1c - r.t0, ns = nstage + r.own;                             // the step's own key and value are one more stage, of one key, outside the ring
         const uint32_t ring = a.off_ring, slots = a.slots, slot_bytes = a.slot_bytes, full = bar_full(a);
-        const float scale = a.scale_log2;
+        
 #pragma unroll 1
         for (int sn = 0; sn < ns; ++sn) {                            // a warp takes 32 keys of its stages
-            const bool in_ring = sn < r.nstage;
+            const bool in_ring = sn < nstage;
             if ((sn & (kStepWarps / kPer - 1)) == warp / kPer) {
-                const int skip = 32 * (warp & (kPer - 1)), n = (in_ring ? r.t1c - r.t0 - sn * kKeys : 1) - skip;
+                const int skip = 32 * (warp & (kPer - 1)), n = (in_ring ? keys - sn * kKeys : 1) - skip;
                 const uint32_t sK = sm0 + (in_ring ? ring + R.slot * slot_bytes : a.off_cur) + skip * 128;
                 if (in_ring) step_wait(R, full + R.bar(), R.par(), 6u);
-                if (n > 0) tile(st, qa, sK, sK + (in_ring ? kHalf : 128), n, scale, g, t);
+                if (n > 0) tile(st, sQ, sK, sK + (in_ring ? kHalf : 128), n, a.scale_log2, g, t);
             }
             if (in_ring) {
                 __syncwarp();
@@ -707,6 +709,14 @@ struct StepLayers {
                     L0 += ml[w].y * f0; L1 += ml[w].w * f1;
                 }
             const int d = ((warp >> 2) * 8 + perm(g)) * 8 + 2 * (warp & 3);
+            if (r.nne == 1) {                                            // the only range: nothing is left to merge
+                const float i0 = __frcp_rn(L0), i1 = __frcp_rn(L1);
+                const __half2 h0 = __floats2half2_rn(acc.x * i0, acc.z * i0), h1 = __floats2half2_rn(acc.y * i1, acc.w * i1);
+                const int at = (r.kvh * grp + 2 * t) * HD + d;
+                if (2 * t < grp) { st_word(a.w_att + at / 2, *reinterpret_cast<const uint32_t*>(&h0), seq); if (last) *reinterpret_cast<__half2*>(a.att + at) = h0; }
+                if (2 * t + 1 < grp) { st_word(a.w_att + (at + HD) / 2, *reinterpret_cast<const uint32_t*>(&h1), seq); if (last) *reinterpret_cast<__half2*>(a.att + at + HD) = h1; }
+                return;
+            }
             if (2 * t < grp) {
                 st_word2(a.w_part + (size_t)slot0 * HD + d, __float_as_uint(acc.x), __float_as_uint(acc.z), seq);
                 if (warp == 0 && g == 0) st_word2(a.w_ml + slot0 * 2, __float_as_uint(M0), __float_as_uint(L0), seq);
@@ -728,15 +738,13 @@ struct StepLayers {
 #pragma unroll 1
         for (int s = warp; s < nne; s += kStepWarps) {
             const int slot = head * a.nsplit + s;
-            uint32_t v[2 * NP], ml[2];
-            poll_words<1>(R, a.w_ml + slot * 2, 0, seq, ml);
-            poll_words<NP>(R, a.w_part + (size_t)slot * HD + lane * ND, 2, seq, v);
-            const float m = __uint_as_float(ml[0]), Mn = fmaxf(M, m);
-            if (Mn == -INFINITY) continue;
+            uint32_t v[2 * NP + 2];                                  // the values, then maximum and sum, in one round trip
+            poll_words<NP, 1>(R, a.w_part + (size_t)slot * HD + lane * ND, 2, a.w_ml + slot * 2, seq, v);
+            const float m = __uint_as_float(v[2 * NP]), Mn = fmaxf(M, m);
             const float fo = M == -INFINITY ? 0.f : ex2(M - Mn), fn = m == -INFINITY ? 0.f : ex2(m - Mn);
 #pragma unroll
             for (int k = 0; k < ND; ++k) acc[k] = acc[k] * fo + __uint_as_float(v[k]) * fn;
-            L = L * fo + __uint_as_float(ml[1]) * fn; M = Mn;
+            L = L * fo + __uint_as_float(v[2 * NP + 1]) * fn; M = Mn;
         }
         consumer_sync(kStepConsumers);                               // every thread has left the merge of this CTA's own partial
         float* o_w = reinterpret_cast<float*>(step_smem + a.off_x);
@@ -779,7 +787,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) step_layers_kernel(const __gr
         mbar_fence_init();
         *reinterpret_cast<typename S::Range*>(step_smem + a.off_range) = S::make_range(a);
     }
-    if (tid < 40) reinterpret_cast<uint32_t*>(step_smem + a.off_zero)[tid] = 0u;
+    if (tid < 64) reinterpret_cast<uint32_t*>(step_smem + a.off_zero)[tid] = 0u;
     if (tid < SP_COUNT * kStepWarps) {
         const int ph = tid / kStepWarps, w = tid % kStepWarps;
         const StepGemv& G = a.g[ph];
@@ -839,7 +847,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) step_layers_kernel(const __gr
         }
         const typename S::Range& rg = S::range(a);
         if (ph == SP_O) {
-            if (rg.any) S::attend(seq, R);
+            if (rg.any) S::attend(seq, l == a.n_layers - 1, R);
             if (rg.fold_head >= 0) S::fold(l, seq, rg.fold_head, R);
         }
         if (rg.nb[ph]) S::gemv(ph, rg.nb[ph], l, seq, R);
