@@ -143,9 +143,14 @@ int launch_delta_rows(const DeltaArgs& a, const LaunchCfg& cfg) {
 struct DeltaTmaps { CUtensorMap qk, v, sc; };
 // CTA: head x CB value channels, NC of them to a thread; four tokens at a time: their products with the state before them are summed over the
 // lanes together, the four corrections follow from the pair products of delta_rows, and the state takes one decay and four updates.
+// What bounds it is the chain from one four tokens to the next, with about one warp a scheduler: so the sixteen sums over a channel pair's lanes are halved level by level (14
+// exchanges for eight lanes, and eight to hand the keys' sums round) instead of every lane summing all (48), and a read-out is finished by the one lane with its sum.  Rows and
+// scan of 28 heads of 128 x 128, a call by itself, 2500 tokens 1050 -> 910 us, 512 tokens 218 -> 192; 12 heads, 2500 tokens 840 -> 710; 64 x 64 within the runs' difference.
+// Twice the lanes to a channel, half the state each, took 912 and 825 us, and 803 instead of 611 where 128 heads fill the chip.
 template <int LPC, int NV, int NC, int CB>
 __global__ void __launch_bounds__(CB / NC * LPC) delta_scan_kernel(const DeltaArgs a, const __grid_constant__ DeltaTmaps m) {
     constexpr int D = LPC * NV * 4, SC = kRecurTile / 4 * kDeltaBlock, STAGE = kRecurTile * (2 * D + CB) + SC;       // q | k | v | block scalars
+    constexpr int LS = LPC < 16 ? LPC : 16, H = 16 / LS;              // lanes that share sixteen sums, sums of a lane
     static_assert(NC == 2, "a thread's channels are one 8-byte unit of a value row");
     extern __shared__ __align__(128) float dr_smem[];   // [2][STAGE]
     __shared__ __align__(8) unsigned long long bars[2];
@@ -167,7 +172,6 @@ __global__ void __launch_bounds__(CB / NC * LPC) delta_scan_kernel(const DeltaAr
     float* st = a.state + ((size_t)h * a.vdimp + c) * a.dimp;         // vdimp is a multiple of eight: both channels exist or none
 #pragma unroll
     for (int j = 0; j < NC; ++j) if (c < a.vdimp && first > 0) s[j].load(st + j * a.dimp, l, a.dimp); else s[j].zero();
-    float* out = a.o + (size_t)l * a.ldo + (size_t)h * a.vdimp + c;
     bool failed = false;
     for (int t0 = 0, i = 0; t0 < a.T; t0 += kRecurTile, ++i) {
         const int b = i & 1;
@@ -177,7 +181,7 @@ __global__ void __launch_bounds__(CB / NC * LPC) delta_scan_kernel(const DeltaAr
 #pragma unroll 1
         for (int tb = 0; tb < n; tb += 4) {
             f32x2 k[4][2 * NV];
-            float sk[4][NC], sq[4][NC];
+            float w[16];                                // 4 t + 2 j + (0: S^T k, 1: S^T q) of token t, channel j
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 f32x2 q[2 * NV];
@@ -187,40 +191,55 @@ __global__ void __launch_bounds__(CB / NC * LPC) delta_scan_kernel(const DeltaAr
                     f32x2 ka = mul2(s[j].s[0], k[t][0]), qa = mul2(s[j].s[0], q[0]);
 #pragma unroll
                     for (int x = 1; x < 2 * NV; ++x) { ka = fma2(s[j].s[x], k[t][x], ka); qa = fma2(s[j].s[x], q[x], qa); }
-                    sk[t][j] = sum2(ka); sq[t][j] = sum2(qa);
+                    w[4 * t + 2 * j] = sum2(ka); w[4 * t + 2 * j + 1] = sum2(qa);
                 }
             }
+            // The sixteen sums over the lanes end up shared out among them, lane l with those from (l mod LS) H on: half of what a lane holds goes to its partner at each level.
 #pragma unroll
-            for (int o = LPC / 2; o > 0; o >>= 1)
+            for (int o = LS / 2, m = 8; o > 0; o >>= 1, m >>= 1)
 #pragma unroll
-                for (int t = 0; t < 4; ++t)
+                for (int i = 0; i < m; ++i) {
+                    const float keep = l & o ? w[m + i] : w[i], send = l & o ? w[i] : w[m + i];
+                    w[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            if (LPC > LS)
 #pragma unroll
-                    for (int j = 0; j < NC; ++j) { sk[t][j] += __shfl_xor_sync(0xffffffffu, sk[t][j], o); sq[t][j] += __shfl_xor_sync(0xffffffffu, sq[t][j], o); }
+                for (int i = 0; i < H; ++i) w[i] += __shfl_xor_sync(0xffffffffu, w[i], LS);
+            const float* cs = cb + (tb >> 2) * kDeltaBlock;
             float x[kDeltaBlock];
 #pragma unroll
             for (int q = 0; q < 7; ++q) {
-                const float4 v = reinterpret_cast<const float4*>(cb + (tb >> 2) * kDeltaBlock)[q];
+                if (q > 3 && q < 6) continue;           // (the read-outs' factors: below)
+                const float4 v = reinterpret_cast<const float4*>(cs)[q];
                 x[4 * q] = v.x; x[4 * q + 1] = v.y; x[4 * q + 2] = v.z; x[4 * q + 3] = v.w;
             }
-            float u[4][NC], o[4][NC];
+            // the corrections, by every lane, from all lanes' sums with the keys
+            float u[4][NC];
             {
-                int ia = 8, ib = 14;
+                int ia = 8;
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
                     const float2 v = *reinterpret_cast<const float2*>(vb + (tb + t) * CB + cg * NC);
 #pragma unroll
                     for (int j = 0; j < NC; ++j) {
-                        float e = (j ? v.y : v.x) - x[t] * sk[t][j];
+                        float e = (j ? v.y : v.x) - x[t] * __shfl_sync(0xffffffffu, w[(4 * t + 2 * j) % H], (4 * t + 2 * j) / H, LPC);
 #pragma unroll
                         for (int p = 0; p < t; ++p) e -= x[ia + p] * u[p][j];
                         u[t][j] = x[4 + t] * e;
-                        float r = x[t] * sq[t][j];
-#pragma unroll
-                        for (int p = 0; p <= t; ++p) r = fmaf(x[ib + p], u[p][j], r);
-                        o[t][j] = r;
                     }
-                    ia += t; ib += t + 1;
+                    ia += t;
                 }
+            }
+            // the read-outs, each by the lane with its sum with the query
+#pragma unroll
+            for (int r = 0; r < H; ++r) {
+                const int e = (l % LS) * H + r, t = e >> 2, j = e >> 1 & 1;
+                if ((H > 1 && r % 2 == 0) || tb + t >= n || c >= a.vdimp || e % 2 == 0 || l >= LS) continue;
+                const float* xb = cs + 14 + t * (t + 1) / 2;
+                float o = cs[t] * w[r];
+#pragma unroll
+                for (int p = 0; p < 4; ++p) if (p <= t) o = fmaf(xb[p], j ? u[p][1] : u[p][0], o);
+                a.o[(size_t)(t0 + tb + t) * a.ldo + (size_t)h * a.vdimp + c + j] = o;
             }
             const f32x2 g2 = pack2(x[3], x[3]);
 #pragma unroll
@@ -236,11 +255,6 @@ __global__ void __launch_bounds__(CB / NC * LPC) delta_scan_kernel(const DeltaAr
                     s[j].s[y] = z;
                 }
             }
-            // lane t of a channel's first four stores token t
-            float2 r = make_float2(o[0][0], o[0][1]);
-#pragma unroll
-            for (int t = 1; t < 4; ++t) { r.x = l == t ? o[t][0] : r.x; r.y = l == t ? o[t][1] : r.y; }
-            if (tb + l < min(n, tb + 4) && c < a.vdimp) *reinterpret_cast<float2*>(out + (size_t)(t0 + tb) * a.ldo) = r;
         }
         __syncthreads();
         if (tid == 0 && t0 + 2 * kRecurTile < a.T) bring(t0 + 2 * kRecurTile, b);
