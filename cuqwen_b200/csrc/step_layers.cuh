@@ -13,13 +13,16 @@
 // residual, gate/up + SwiGLU, down projection + residual.  A CTA keeps the residual of its own rows in shared memory (the two row-parallel projections are cut
 // alike).  CTAs without work in a phase do not read its input.
 //
-// Measured, us a step, launch by launch -> here (one B200, the same box): 0.5B int4 at 255 keys 677 -> 439, 0.5B fp16 at 1777 655 -> 523, 7B int4 at 8192 1462 -> 1230, six 14B int8 layers
-// at 31,999 691 -> 638.  What the phases take, in cycles of 1.85 GHz (0.5B int4 / 7B int4): hand-over 1300 / 1400 to 2000; a vector to digits 400 / 750 and its norm 250; products
-// 1300 / 3100 (q/k/v, o), 18,600 (7B gate/up, 70 MB), 12,800 (down); a block's finish 900 to 1500; attention 3700 / 9500, of which a tile of 32 keys is 790 / 1500; merge of the
-// partials 2300 / 7000.  The 7B layer's bytes alone would take 39,000 of its 78,000 cycles.
+// Measured, us a step, launch by launch -> here (one B200, the same box): 0.5B int4 at 255 keys 677 -> 434, 0.5B fp16 at 1777 655 -> 498, 7B int4 at 8192 1462 -> 1104, six 14B int8 layers
+// at 31,999 691 -> 603.  What the phases take, in cycles of 1.9 GHz (0.5B int4 / 7B int4): hand-over, from one phase's end until its words are here, 2000 / 2000 to 2500; a vector to digits
+// 370 / 740 and its norm 250; products 1150 / 2780 (q/k/v), 16,800 (7B gate/up, 70 MB), 11,600 (down); a block's finish 800 to 1300; attention 6400 / 7300, of which the tile loop
+// 2800 / 3800; merge of the partials, 7B, 5500 to 8500.  The 7B layer's bytes alone would take 39,000 of its 69,000 cycles.
+// A warp's products of one group cost some 600 cycles next to the fifteen other warps' (operands from shared memory 390 and the integer MMAs 300), a chain, not a rate.  Slower were: the next
+// group's weights loaded ahead (7B 1094 -> 1240 us), two groups side by side (1173), rolled loops in the attention (1100 to 1135), a head's merge shared out among the CTAs that it has (1128),
+// polls through one lane a warp (1160) and weights asked into L2 ahead of the ring (1210).
 //
 // What this cost most to find: the consumers' code must fit the instruction caches (118 KB of phases inlined four times took 40 us a layer of the 0.5B model, 60 KB with one copy of
-// the phases 19), no register may spill (the spill lines' L1 is what 227 KB of shared memory leave, 28 KB; the 14B step 708 -> 637 us when the spills went), and keys and values
+// the phases 19), no register may spill (the spill lines' L1 is what 227 KB of shared memory leave, 28 KB; the 14B step 708 -> 637 us when most of them went), and keys and values
 // must not collide in the banks (a tile 2300 -> 1500 cycles).
 #pragma once
 #include "attn_split.cuh"
@@ -849,6 +852,8 @@ __global__ void __launch_bounds__(kStepThreads, 1) step_layers_kernel(const __gr
         if (ph == SP_O) {
             if (rg.any) S::attend(seq, l == a.n_layers - 1, R);
             if (rg.fold_head >= 0) S::fold(l, seq, rg.fold_head, R);
+            // Both end with a few warps reading the area that the output projection's input is staged in, whose first words may be other heads'.
+            if (rg.any || rg.fold_head >= 0) consumer_sync(kStepConsumers);
         }
         if (rg.nb[ph]) S::gemv(ph, rg.nb[ph], l, seq, R);
     }
