@@ -169,7 +169,7 @@ def dominant_kernel_roofline(eng, E, K, model_cfg, quant_id: int, iters: int = 2
     wbytes = eng.ptr("WGATE", 0)[1] + eng.ptr("SGATE", 0)[1]
     eps = float(np.float16(1e-6))               # the reference narrows eps to fp16 (src/model.cu:131-134)
 
-    def sweep():      # the kernel exactly as the step launches it: fused RMSNorm prologue with the layer's own weight
+    def sweep():      # the phase as a kernel of its own (a step of separate launches runs it so): fused RMSNorm prologue with the layer's own weight
         for wg, wu, sg, su, nw in ptrs:
             K.fused_mlp_stage1(quant_id, x, wg, wu, sg, su, out, dim, inter_l, norm_weight=nw, eps=eps, device=eng.device)
 
