@@ -831,6 +831,9 @@ __global__ void __launch_bounds__(kStepThreads, 1) step_layers_kernel(const __gr
             S::qkv_tile(a, (int)(blockIdx.x + j * gridDim.x), mat, row);
             if (tid < 16) { float c, s; rope_cs((row + tid) % HD, HD, S::range(a).pos, a.theta, 1, &c, &s); rope[j * 16 + tid] = make_float2(c, s); }
         }
+        // Both arrays are written by the first warps and read by the threads that finish a row, of up to four warps, before any other barrier: the rotation when layer 0's
+        // q/k/v phase begins, the residual in a CTA whose first work is the output projection.
+        consumer_sync(kStepConsumers);
     }
     StepRing R{0u, 0u, 0u, 0u, 0u};
     const uint32_t seq0 = *a.epoch * kSeqPerStep;

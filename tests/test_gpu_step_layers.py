@@ -125,3 +125,34 @@ def test_the_same_step_again(built, tmp_path, quant, heads, kv, hd, ctx):
         e.step(5, ctx)
         assert np.array_equal(e.read("LOGITS").view(np.uint16), first.view(np.uint16)), i
     e.close()
+
+
+@pytest.mark.parametrize("dim,inter,heads,kv,hd", [(896, 4864, 14, 2, 64), (1536, 8960, 12, 2, 128), (2048, 11008, 16, 2, 128)])
+@pytest.mark.parametrize("quant", [0, 1, 2])
+def test_steps_at_changing_places(built, tmp_path, quant, dim, inter, heads, kv, hd):
+    """What a CTA prepares before the first layer, the rotation and its rows of the residual stream, is the step's own: tokens and positions that jump from step to step, up to 256 keys (many CTAs
+    begin with the output projection) and beyond.  Layer 0's key row and the logits are those of the separate launches (bound: see above), and a step's bits do not depend on the step before
+    it (each runs over the same cached rows in both orders)."""
+    cfg = dict(vocab=512, dim=dim, inter=inter, layers=2, heads=heads, kv=kv, hd=hd, tied=True)
+    path = tmp_path / "m.bin"
+    binfmt.write_model(path, cfg, quant, binfmt.random_tensors(cfg, 5))
+    a, b = make(cfg, quant, path), make(cfg, quant, path, E.FLAG_NO_HANDOVER)
+    rng = np.random.default_rng(3)
+    places = [(int(rng.integers(512)), int(rng.integers(*r))) for _ in range(20) for r in ((0, 256), (256, MAX_SEQ))]
+
+    def run(e, tok, pos):
+        e.kv_fill_normal(pos, 7)
+        e.step(tok, pos)
+        return e.read("LOGITS"), e.read("KEY_CACHE").reshape(2, kv, MAX_SEQ, hd)[0, :, pos]
+
+    first = [run(a, *p) for p in places]
+    assert a.step_launches == 5
+    for p, got in zip(places, first):
+        for g, w in zip(got, run(b, *p)):
+            g, w = g.astype(np.float64), w.astype(np.float64)
+            assert np.linalg.norm(g - w) <= 5e-3 * np.linalg.norm(w), p
+    for i in np.random.default_rng(4).permutation(len(places)):
+        for g, w in zip(run(a, *places[i]), first[i]):
+            assert np.array_equal(g.view(np.uint16), w.view(np.uint16)), places[i]
+    a.close()
+    b.close()
