@@ -583,25 +583,24 @@ struct StepLayers {
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {        // keys 16h .. 16h + 15: one k-step of P.V, in the order of the scores
-            uint4 vv[4][NC];
+            // 64 columns at a time: all of a row's fragments at once are 16 registers more, and what other phases keep in registers then spills (fp16 with heads of 128, us a step with 40 and with 0
+            // bytes spilled: eight layers of 1.5B at 3000 keys 356 -> 324, six of 3B 371 -> 340, four of 7B 540 -> 519, where the separate launches take 346, 355 and 518).
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
+            for (int c = 0; c < NC; ++c) {
+                uint4 vv[4];
 #pragma unroll
-                for (int c = 0; c < NC; ++c) vv[r][c] = lds128((r & 1 ? v1 : v0) + c * COLS + h * 2048 + (r >> 1) * 1024);
-            if (n < 16 * h + 16) {           // a row that does not exist may hold anything: its weight is 0, and 0 times that must be 0
+                for (int r = 0; r < 4; ++r) vv[r] = lds128((r & 1 ? v1 : v0) + c * COLS + h * 2048 + (r >> 1) * 1024);
+                if (n < 16 * h + 16) {       // a row that does not exist may hold anything: its weight is 0, and 0 times that must be 0
 #pragma unroll
-                for (int r = 0; r < 4; ++r)
-                    if (16 * h + 8 * (r >> 1) + t + 4 * (r & 1) >= n)
-#pragma unroll
-                        for (int c = 0; c < NC; ++c) vv[r][c] = make_uint4(0u, 0u, 0u, 0u);
-            }
-#pragma unroll
-            for (int c = 0; c < NC; ++c)
+                    for (int r = 0; r < 4; ++r)
+                        if (16 * h + 8 * (r >> 1) + t + 4 * (r & 1) >= n) vv[r] = make_uint4(0u, 0u, 0u, 0u);
+                }
 #pragma unroll
                 for (int ep = 0; ep < 4; ++ep) {
-                    const uint32_t wA = u4c(vv[0][c], ep), wB = u4c(vv[1][c], ep), wC = u4c(vv[2][c], ep), wD = u4c(vv[3][c], ep);
+                    const uint32_t wA = u4c(vv[0], ep), wB = u4c(vv[1], ep), wC = u4c(vv[2], ep), wD = u4c(vv[3], ep);
                     mma16816(st.o[c * 4 + ep], prmt(wA, wB, 0x5410), prmt(wA, wB, 0x7632), prmt(wC, wD, 0x5410), prmt(wC, wD, 0x7632), pb[2 * h], pb[2 * h + 1]);
                 }
+            }
         }
     }
 

@@ -1,7 +1,9 @@
 """Which engines run a step's layers as one kernel, and which launch by launch, on the CPU over tests/cudart_stub.cpp."""
+import re
+
 import pytest
 
-from cuqwen_b200 import binfmt
+from cuqwen_b200 import binfmt, build
 from test_host_memory import run                                           # noqa: F401  (fixture)
 
 PLAIN = dict(vocab=512, dim=256, inter=512, layers=2, heads=4, kv=2, hd=64, tied=True)
@@ -36,3 +38,12 @@ def test_the_layers_of_a_step_are_one_launch(run, tmp_path, quant, hd):     # no
                                               ("0", 75, 148), ("0", 0, 3)])
 def test_what_the_kernel_does_not_know_stays_launch_by_launch(run, tmp_path, flags, splits, sms):      # noqa: F811
     assert "step_layers_kernel" not in kernels_of_a_step(run, tmp_path, PLAIN, 2, flags, splits, sms)
+
+
+def test_no_variant_spills():
+    """A spilled register costs the step up to a tenth (fp16 with heads of 128: slower than the separate launches): its line is not in the little L1 that the kernel's shared memory leaves."""
+    logs = [build.OBJ / f"step_layers_{q}.ptxas.txt" for q in ("i4", "i8", "f16")]
+    if not all(p.exists() for p in logs):
+        pytest.skip("the library was not built here")
+    spills = re.findall(r"(\d+) bytes spill stores, (\d+) bytes spill loads", "".join(p.read_text() for p in logs))
+    assert spills == [("0", "0")] * 6
