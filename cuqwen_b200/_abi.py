@@ -48,6 +48,7 @@ SIGNATURES = {
     "cuqwen_get_params": (_i, [_vp, C.POINTER(Params)]),
     "cuqwen_step_bytes": (C.c_uint64, [_vp, _i]),
     "cuqwen_step_launches": (_i, [_vp]),
+    "cuqwen_set_wait_cycles": (_i, [_vp, C.c_uint32]),
     "cuqwen_step_profile": (_i, [_vp, _i, _i, C.POINTER(C.c_float), _i, C.POINTER(_i)]),
     "cuqwen_dev_alloc": (_i, [_i, _sz, C.POINTER(_vp)]),
     "cuqwen_dev_sm_count": (_i, [_i, _pi]),

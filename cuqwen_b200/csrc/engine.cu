@@ -410,7 +410,7 @@ static int prepare_layers(cuqwen_engine* e) {
     for (int i = 0; i < SM_COUNT; ++i) c.scale[i] = m[i]->s;
     c.bias[0] = L.bq; c.bias[1] = L.bk; c.bias[2] = L.bv; c.norm[0] = L.in_norm; c.norm[1] = L.post_norm;
     c.x = e->x; c.q = e->q; c.k = e->k; c.v = e->v; c.att = e->att; c.gate = e->gate; c.kc = e->kc; c.vc = e->vc;
-    c.d_pos = &e->ctl->pos; c.err = reinterpret_cast<unsigned*>(&e->ctl->pad[0]);
+    c.d_pos = &e->ctl->pos; c.err = reinterpret_cast<unsigned*>(&e->ctl->pad[0]); c.wait_cycles = kStepWaitCycles;
     c.eps = __half2float(__float2half(p.norm_eps)); c.scale_log2 = (1.0f / sqrtf((float)p.head_dim)) * 1.4426950408889634f; c.theta = p.rope_theta;
     for (size_t& n : words) { n = align_up(n, 16); total += n; }
     if (cudaMalloc((void**)&e->layers_words, total * 8 + 128) != cudaSuccess) { cudaGetLastError(); e->layers_words = nullptr; return CUQWEN_OK; }
@@ -1073,6 +1073,18 @@ extern "C" int cuqwen_tp_plan(int n_heads, int n_kv, int hd, int inter, int voca
 
 extern "C" int cuqwen_lm_head_kind(const cuqwen_engine* e) { return e ? e->lm_kind : -1; }
 extern "C" int cuqwen_get_params(const cuqwen_engine* e, cuqwen_params* out) { if (!e || !out) return fail(CUQWEN_ERR_ARG, "null argument"); *out = e->p; out->attn_splits = e->nsplit; return CUQWEN_OK; }
+extern "C" int cuqwen_set_wait_cycles(cuqwen_engine* e, unsigned cycles) {
+    if (!e) return fail(CUQWEN_ERR_ARG, "null engine");
+    if (!e->layers_args) return fail(CUQWEN_ERR_STATE, "this engine's step is launched kernel by kernel");
+    if (cycles > kStepWaitCycles) return fail(CUQWEN_ERR_ARG, "at most %u cycles", kStepWaitCycles);
+    CK(cudaSetDevice(e->p.device));
+    CK(cudaStreamSynchronize(e->stream));
+    e->layers_args->c.wait_cycles = cycles ? cycles : kStepWaitCycles;
+    if (e->gexec) cudaGraphExecDestroy(e->gexec);          // the graph holds the arguments: the next step captures it anew
+    if (e->graph) cudaGraphDestroy(e->graph);
+    e->gexec = nullptr; e->graph = nullptr; e->graph_ready = false;
+    return CUQWEN_OK;
+}
 extern "C" int cuqwen_step_launches(const cuqwen_engine* e) { return e ? e->launches : 0; }
 extern "C" uint64_t cuqwen_step_bytes(const cuqwen_engine* e, int ctx) {
     if (!e) return 0;

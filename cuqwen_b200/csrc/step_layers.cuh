@@ -59,27 +59,41 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
 struct StepRing {
     uint32_t n, slot;                // next stage, its slot
     uint32_t red;                    // which of the two buffers of the warps' sums comes next
-    uint32_t failed, poll_failed;    // code of a wait on the ring / on words that expired: that kind of wait is over for this thread
     __device__ __forceinline__ uint32_t bar() const { return (n & (kStepBars - 1)) * 8; }
     __device__ __forceinline__ uint32_t par() const { return (n / kStepBars) & 1u; }
     __device__ __forceinline__ void next(uint32_t slots) { ++n; if (++slot == slots) slot = 0; }
-    __device__ __forceinline__ void report(unsigned* err) const { if (err && (failed | poll_failed)) atomicExch(err, failed ? failed : poll_failed); }
 };
 __device__ __forceinline__ uint32_t cycles32() { uint32_t t; asm volatile("mov.u32 %0, %clock;" : "=r"(t)); return t; }
-// Bounded, as every wait, here by 2e9 cycles (about a second), in few instructions: the layers' code has to stay in the instruction cache.
-__device__ __forceinline__ void step_wait(StepRing& R, uint32_t bar, uint32_t parity, unsigned code) {
-    if (mbar_try_wait(bar, parity) || R.failed) return;
-    const uint32_t t0 = cycles32();
+
+// Shared memory of a CTA; the argument block lies at its start, where the consumers' phases read it: read from the parameters, the compiler carries the phases' constants
+// through all layers, in registers that sixteen warps (112 a thread) do not have.
+extern __shared__ __align__(1024) unsigned char step_smem[];
+
+// Every wait, on the ring or on words, is over when the CTA has run for StepCore::wait_cycles (a step takes some thousandth of the default; a start of its own for every wait would cost a
+// register).  The first one that ends so leaves its code in the CTA's argument block, and from then on every wait of the CTA ends at its first look: the CTA goes through the rest of the
+// step at once, with whatever its memory holds (no value decides an address), and hands on the words that the other CTAs wait for.  The producer begins no copy after that; those
+// under way: see land.
+__device__ __forceinline__ uint32_t lds_volatile(uint32_t at) { uint32_t v; asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(step_smem) + at)); return v; }
+__device__ __forceinline__ uint32_t step_expired() { return lds_volatile(offsetof(StepCore, expired)); }
+__device__ __forceinline__ bool step_expire(uint32_t code) {
+    if (step_expired()) return true;
+    if (cycles32() - lds_volatile(offsetof(StepCore, started)) <= lds_volatile(offsetof(StepCore, wait_cycles))) return false;
+    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(smem_u32(step_smem) + (uint32_t)offsetof(StepCore, expired)), "r"(code));
+    return true;
+}
+__device__ __forceinline__ void step_report(unsigned* err) { if (const uint32_t code = step_expired()) atomicExch(err, code); }
+// In few instructions: the layers' code has to stay in the instruction cache.
+__device__ __forceinline__ void step_wait(uint32_t bar, uint32_t parity, uint32_t code) {
+    if (mbar_try_wait(bar, parity)) return;
 #pragma unroll 1
     while (!mbar_try_wait(bar, parity))
-        if (cycles32() - t0 > 2000000000u) { R.failed = code; return; }
+        if (step_expire(code)) return;
 }
-// Polls N pairs of words, `stride` words apart, and (EXTRA) the pair at q, until all carry `seq`; bounded by 2^20 tries of an L2 round trip each (some 0.3 s: less than the ring's limit, which therefore does
-// not expire with it); after that the thread polls no more in this step.  The ring goes on, so that no copy is under way when the CTA ends.
+// Polls N pairs of words, `stride` words apart, and (EXTRA) the pair at q, until all carry `seq`.
 template <int N, int EXTRA = 0>
-__device__ __forceinline__ void poll_words(StepRing& R, const uint2* p, int stride, const uint2* q, uint32_t seq, uint32_t (&v)[2 * (N + EXTRA)]) {
+__device__ __forceinline__ void poll_words(const uint2* p, int stride, const uint2* q, uint32_t seq, uint32_t (&v)[2 * (N + EXTRA)]) {
 #pragma unroll 1
-    for (int tries = 1 << 20;; --tries) {
+    for (;;) {
         uint32_t bad = 0;
         unsigned long long a[N + EXTRA], b[N + EXTRA];
 #pragma unroll
@@ -87,16 +101,11 @@ __device__ __forceinline__ void poll_words(StepRing& R, const uint2* p, int stri
         if (EXTRA) ld_word2(q, a[N + EXTRA - 1], b[N + EXTRA - 1]);
 #pragma unroll
         for (int i = 0; i < N + EXTRA; ++i) { v[2 * i] = (uint32_t)a[i]; v[2 * i + 1] = (uint32_t)b[i]; bad |= ((uint32_t)(a[i] >> 32) ^ seq) | ((uint32_t)(b[i] >> 32) ^ seq); }
-        if (bad == 0 || R.poll_failed) return;
-        if (tries == 0) R.poll_failed = 11u;
+        if (bad == 0 || step_expire(11u)) return;
     }
 }
 template <int N>
-__device__ __forceinline__ void poll_words(StepRing& R, const uint2* p, int stride, uint32_t seq, uint32_t (&v)[2 * N]) { poll_words<N, 0>(R, p, stride, nullptr, seq, v); }
-
-// Shared memory of a CTA; the argument block lies at its start, where the consumers' phases read it: read from the parameters, the compiler carries the phases' constants
-// through all layers, in registers that sixteen warps (112 a thread) do not have.
-extern __shared__ __align__(1024) unsigned char step_smem[];
+__device__ __forceinline__ void poll_words(const uint2* p, int stride, uint32_t seq, uint32_t (&v)[2 * N]) { poll_words<N, 0>(p, stride, nullptr, seq, v); }
 
 template <int Q, int HD>
 struct StepLayers {
@@ -131,15 +140,28 @@ struct StepLayers {
     static constexpr int kDirect = 256;
     // A free slot for the next stage, whose barrier then expects `tx` bytes.  One thread issues all copies of an SM, some 40 instructions a stage
     // (slots of one size: with stages packed behind one another it took 90, and was what the large matrices waited for).
-    static __device__ __forceinline__ uint32_t claim(StepRing& R, uint32_t full, uint32_t slots, uint32_t tx) {
+    // 0: a wait of this CTA has expired.  That is looked up behind the wait, which may have ended because warps let stages go that they had not waited for.
+    static __device__ __forceinline__ uint32_t claim(const StepRing& R, uint32_t full, uint32_t slots, uint32_t tx) {
         const uint32_t before = R.n - slots;                // the stage that had the slot
-        if (R.n >= slots) step_wait(R, full + (kStepBars + (before & (kStepBars - 1))) * 8, (before / kStepBars) & 1u, 4u);
+        if (R.n >= slots) step_wait(full + (kStepBars + (before & (kStepBars - 1))) * 8, (before / kStepBars) & 1u, 4u);
+        if (step_expired()) return 0u;
         const uint32_t bar = full + R.bar();
-        if (!R.failed) mbar_expect_tx(bar, tx);
+        mbar_expect_tx(bar, tx);
         return bar;
     }
-    // No copy is begun after an expired wait: it could land in a stage that is still read.
-    static __device__ __forceinline__ void produce_gemv(const StepArgs& args, StepRing& R, int ph, int l, int nb) {
+    // Before the CTA ends, also early: the last copies announced by each barrier have arrived, as none may land in the shared memory of a CTA that comes after this one.  Bounded as a
+    // step's waits are by default, whatever this step's are.
+    static __device__ __forceinline__ void land(const StepCore& a, const StepRing& R, uint32_t scales) {
+        const uint32_t full = bar_full(a), t0 = cycles32();
+#pragma unroll 1
+        for (uint32_t n = R.n > kStepBars ? R.n - kStepBars : 0u; n < R.n; ++n)
+            while (!mbar_try_wait(full + (n & (kStepBars - 1)) * 8, (n / kStepBars) & 1u) && cycles32() - t0 <= kStepWaitCycles) {}
+#pragma unroll 1
+        for (int ph = 0; ph < SP_COUNT; ++ph)
+            while (scales >> (8 + ph) & 1u && !mbar_try_wait(bar_sfull(a, ph), scales >> ph & 1u) && cycles32() - t0 <= kStepWaitCycles) {}
+    }
+    // false: see claim.  scales: which phases' scale barriers were armed (bits 8 ..) and the parity of their last use (bits 0 ..)
+    static __device__ __forceinline__ bool produce_gemv(const StepArgs& args, StepRing& R, int ph, int l, int nb, uint32_t& scales) {
         const StepCore& a = args.c;
         const StepGemv& G = a.g[ph];
         const uint32_t sm0 = smem_u32(step_smem), ring = sm0 + a.off_ring, full = bar_full(a), slots = a.slots, slot_bytes = a.slot_bytes;
@@ -147,12 +169,13 @@ struct StepLayers {
         const int mt = qkv || ph == SP_MLP ? 2 : 1, m0 = ph == SP_O ? SM_O : ph == SP_MLP ? SM_GATE : SM_DOWN, ngrp = G.ngrp;
         if (kInt) {
             // the scales of all of the phase's blocks before the first stage: the consumers wait for them once, and the ring need not hold a whole block
-            step_wait(R, bar_sempty(a, ph), (l & 1) ^ 1, 3u);
+            step_wait(bar_sempty(a, ph), (l & 1) ^ 1, 3u);
             uint32_t total = 0;
 #pragma unroll 1
             for (int j = 0; j < nb; ++j) total += (uint32_t)(mt * ngrp * 2) * (qkv ? 16 : min(G.brows, G.rows - (int)(blockIdx.x + j * gridDim.x) * G.brows));
-            if (R.failed) return;
+            if (step_expired()) return false;
             mbar_expect_tx(bar_sfull(a, ph), total);
+            scales = (scales & ~(1u << ph)) | 256u << ph | (uint32_t)(l & 1) << ph;
         }
 #pragma unroll 1
         for (int j = 0; j < 2 * nb; ++j) {                  // scales, then stages
@@ -175,13 +198,14 @@ struct StepLayers {
 #pragma unroll 1
             for (int p = 0; p < nst; ++p) {
                 const uint32_t bar = claim(R, full, slots, tx), dst = ring + R.slot * slot_bytes;
-                if (R.failed) return;
+                if (!bar) return false;
                 tma_load_4d(dst, map0, 0, row, z, l, bar);
                 if (mt == 2) tma_load_4d(dst + box, map1, 0, row + drow, z, l, bar);
                 z += dz;
                 R.next(slots);
             }
         }
+        return true;
     }
     // cached keys and values of this CTA's key range: rows below `pos`, which earlier steps wrote
     static __device__ __forceinline__ Range make_range(const StepCore& a) {
@@ -202,19 +226,20 @@ struct StepLayers {
         for (int i = 0; i < SP_COUNT; ++i) r.nb[i] = cta < a.g[i].nblk ? (a.g[i].nblk - cta + (int)gridDim.x - 1) / (int)gridDim.x : 0;
         return r;
     }
-    static __device__ __forceinline__ void produce_kv(const StepArgs& args, StepRing& R, int l, const Range& r) {
+    static __device__ __forceinline__ bool produce_kv(const StepArgs& args, StepRing& R, int l, const Range& r) {
         const StepCore& a = args.c;
         const uint32_t sm0 = smem_u32(step_smem), ring = sm0 + a.off_ring, full = bar_full(a), slots = a.slots, slot_bytes = a.slot_bytes;
         int row = (l * a.n_kv + r.kvh) * a.max_seq + r.t0;          // rows past the range's end come along and are not used
 #pragma unroll 1
         for (int sn = 0; sn < r.nstage; ++sn) {
             const uint32_t bar = claim(R, full, slots, 2 * kHalf), dst = ring + R.slot * slot_bytes;
-            if (R.failed) return;
+            if (!bar) return false;
             tma_load_3d(dst, &args.kv[0], 0, row, 0, bar);
             tma_load_3d(dst + kHalf, &args.kv[1], 0, row, 0, bar);
             row += kKeys;
             R.next(slots);
         }
+        return true;
     }
 
     // ---- consumers ----------------------------------------------------------
@@ -251,7 +276,7 @@ struct StepLayers {
     // The phase's input vector into shared memory, in the form the products want: from words of two halves (src), or plain (x of the first layer).
     // Quantised weights: a warp takes a group (two at a time, so that their loads overlap).  A norm's 1 / rms is not waited for: the digits are those of x * weight in fp32, and
     // the rows' sums are multiplied by it (norm_scale), which spares a barrier and a rounding to fp16.
-    static __device__ __forceinline__ void stage_vec(StepRing& R, const uint2* src, const __half* plain, const __half* norm_w, int K, uint32_t seq) {
+    static __device__ __forceinline__ void stage_vec(const uint2* src, const __half* plain, const __half* norm_w, int K, uint32_t seq) {
         const StepCore& a = core();
         const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
         float* rms = reinterpret_cast<float*>(step_smem + a.off_rms);
@@ -268,7 +293,7 @@ struct StepLayers {
                 uint32_t v[4];
                 if (norm_w) { const uint2* n = reinterpret_cast<const uint2*>(norm_w) + grp * 32 + lane; w0 = __ldg(n); w1 = __ldg(n + to2); }
                 if (plain) { const uint2* x = reinterpret_cast<const uint2*>(plain) + grp * 32 + lane; const uint2 p = __ldcg(x), q = __ldcg(x + to2); v[0] = p.x; v[1] = p.y; v[2] = q.x; v[3] = q.y; }
-                else poll_words<2>(R, src + grp * 64 + 2 * lane, 2 * to2, seq, v);
+                else poll_words<2>(src + grp * 64 + 2 * lane, 2 * to2, seq, v);
 #pragma unroll 1
                 for (int i = 0; i <= two; ++i) {
                     const uint32_t u0 = i ? v[2] : v[0], u1 = i ? v[3] : v[1], n0 = i ? w1.x : w0.x, n1 = i ? w1.y : w0.y;
@@ -289,7 +314,7 @@ struct StepLayers {
                 if (plain) v = __ldcg(reinterpret_cast<const uint4*>(plain) + c8);
                 else {
                     uint32_t w[4];
-                    poll_words<2>(R, src + c8 * 4, 2, seq, w);
+                    poll_words<2>(src + c8 * 4, 2, seq, w);
                     v = make_uint4(w[0], w[1], w[2], w[3]);
                 }
                 xs[c8] = v;
@@ -315,7 +340,7 @@ struct StepLayers {
         return rsqrtf(s * a.inv_dim + a.eps);
     }
     // The SwiGLU output in staged form: 64 words of digits a group, then correction and scale of each.
-    static __device__ __forceinline__ void stage_groups(StepRing& R, const uint2* src, int ngrp, uint32_t seq) {
+    static __device__ __forceinline__ void stage_groups(const uint2* src, int ngrp, uint32_t seq) {
         constexpr int NB = 5;
         const StepCore& a = core();
         const int n = ngrp * 32, tid = threadIdx.x;
@@ -326,14 +351,14 @@ struct StepLayers {
         for (int u = tid;; u += NB * kStepConsumers) {
             const int over = u + (NB - 1) * kStepConsumers - (n - kStepConsumers + tid);
             if (over > 0) u -= over;
-            poll_words<NB>(R, src + 2 * u, 2 * kStepConsumers, seq, v);
+            poll_words<NB>(src + 2 * u, 2 * kStepConsumers, seq, v);
 #pragma unroll
             for (int i = 0; i < NB; ++i) xd[u + i * kStepConsumers] = make_uint2(v[2 * i], v[2 * i + 1]);
             if (over >= 0) break;
         }
         if (tid < ngrp) {
             uint32_t c[2];
-            poll_words<1>(R, src + 2 * (n + tid), 0, seq, c);
+            poll_words<1>(src + 2 * (n + tid), 0, seq, c);
             reinterpret_cast<uint2*>(step_smem + a.off_corr)[tid] = make_uint2(c[0], c[1]);
         }
         consumer_sync(kStepConsumers);
@@ -373,7 +398,7 @@ struct StepLayers {
         for (int p = 0; p < W.nst; ++p) {
             uint32_t w0 = W.in_stage + R.slot * W.slot_bytes + W.part * W.ustride;
             const uint32_t bar = W.full + R.bar();
-            step_wait(R, bar, R.par(), 1u);
+            step_wait(bar, R.par(), 1u);
             const int n = u0 + min(W.units, left);
 #pragma unroll 1
             for (int grp = u0 + W.part; grp < n; grp += W.kp) {
@@ -463,12 +488,12 @@ struct StepLayers {
                 }
             }
             if (j == 0) {
-                if (kInt) step_wait(R, bar_sfull(a, ph), l & 1, 2u);
-                if (kInt && ph == SP_DOWN && a.staged_h) stage_groups(R, a.w_h, G.ngrp, seq);
+                if (kInt) step_wait(bar_sfull(a, ph), l & 1, 2u);
+                if (kInt && ph == SP_DOWN && a.staged_h) stage_groups(a.w_h, G.ngrp, seq);
                 else {
                     const uint2* src = ph == SP_QKV ? a.w_x2 : ph == SP_O ? a.w_att : ph == SP_MLP ? a.w_x1 : a.w_h;
                     const __half* norm = ph == SP_QKV ? at_layer(a, a.norm[0], l) : ph == SP_MLP ? at_layer(a, a.norm[1], l) : nullptr;
-                    stage_vec(R, src, ph == SP_QKV && l == 0 ? a.x : nullptr, norm, G.K, ph == SP_QKV ? seq - 1 : seq);
+                    stage_vec(src, ph == SP_QKV && l == 0 ? a.x : nullptr, norm, G.K, ph == SP_QKV ? seq - 1 : seq);
                 }
             }
             float tot[2];
@@ -621,7 +646,7 @@ struct StepLayers {
                 const int u = isq ? tid : isk ? j : j - HD / 4;                     // pair inside the heads' / the head's words
                 const int h0 = isq ? r.kvh * grp : (isk ? a.n_heads : a.n_heads + a.n_kv) + r.kvh;
                 uint32_t v[2];
-                poll_words<1>(R, a.w_qkv + h0 * (HD / 2) + 2 * u, 0, seq, v);
+                poll_words<1>(a.w_qkv + h0 * (HD / 2) + 2 * u, 0, seq, v);
                 const int hl = 2 * u / (HD / 2), d = 2 * u - hl * (HD / 2);
                 unsigned char* o = isq ? qs + hl * kRowQ + d * 2 : sm + a.off_cur + (isk ? 0 : 128) + d * 2;
                 *reinterpret_cast<uint32_t*>(o) = prmt(v[0], v[1], 0x5410);
@@ -643,7 +668,7 @@ struct StepLayers {
             if ((sn & (kStepWarps / kPer - 1)) == warp / kPer) {
                 const int skip = 32 * (warp & (kPer - 1)), n = (in_ring ? keys - sn * kKeys : 1) - skip;
                 const uint32_t sK = sm0 + (in_ring ? ring + R.slot * slot_bytes : a.off_cur) + skip * 128;
-                if (in_ring) step_wait(R, full + R.bar(), R.par(), 6u);
+                if (in_ring) step_wait(full + R.bar(), R.par(), 6u);
                 if (n > 0) tile(st, sQ, sK, sK + (in_ring ? kHalf : 128), n, a.scale_log2, g, t);
             }
             if (in_ring) {
@@ -731,7 +756,7 @@ struct StepLayers {
     }
 
     // Merge of a head's partials: warp w takes splits w, w + 16, ..., a lane HD / 32 columns.
-    static __device__ __forceinline__ void fold(int l, uint32_t seq, int head, StepRing& R) {
+    static __device__ __forceinline__ void fold(int l, uint32_t seq, int head) {
         constexpr int ND = HD / 32, NP = ND / 2;
         const StepCore& a = core();
         const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -741,7 +766,7 @@ struct StepLayers {
         for (int s = warp; s < nne; s += kStepWarps) {
             const int slot = head * a.nsplit + s;
             uint32_t v[2 * NP + 2];                                  // the values, then maximum and sum, in one round trip
-            poll_words<NP, 1>(R, a.w_part + (size_t)slot * HD + lane * ND, 2, a.w_ml + slot * 2, seq, v);
+            poll_words<NP, 1>(a.w_part + (size_t)slot * HD + lane * ND, 2, a.w_ml + slot * 2, seq, v);
             const float m = __uint_as_float(v[2 * NP]), Mn = fmaxf(M, m);
             const float fo = M == -INFINITY ? 0.f : ex2(M - Mn), fn = m == -INFINITY ? 0.f : ex2(m - Mn);
 #pragma unroll
@@ -780,7 +805,8 @@ __global__ void __launch_bounds__(kStepThreads, 1) step_layers_kernel(const __gr
     const StepCore& a = args.c;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_launch_dependents();
-    if (tid < (int)(sizeof(StepCore) / 4)) reinterpret_cast<uint32_t*>(step_smem)[tid] = reinterpret_cast<const uint32_t*>(&a)[tid];
+    if (tid < (int)(sizeof(StepCore) / 4))
+        reinterpret_cast<uint32_t*>(step_smem)[tid] = tid == (int)(offsetof(StepCore, started) / 4) ? cycles32() : tid == (int)(offsetof(StepCore, seq0) / 4) ? *a.epoch * kSeqPerStep : reinterpret_cast<const uint32_t*>(&a)[tid];
     if (tid == 0) {
 #pragma unroll 1
         for (int i = 0; i < kStepBars; ++i) { mbar_init(S::bar_full(a) + i * 8, 1); mbar_init(S::bar_empty(a) + i * 8, kStepWarps); }
@@ -801,15 +827,17 @@ __global__ void __launch_bounds__(kStepThreads, 1) step_layers_kernel(const __gr
     if (warp >= kStepWarps) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
         if (warp == kStepWarps && lane == 0) {
-            StepRing P{0u, 0u, 0u, 0u, 0u};
+            StepRing P{0u, 0u, 0u};
             const typename S::Range& rg = S::range(a);
+            uint32_t scales = 0u;
 #pragma unroll 1
-            for (int i = 0; i < a.n_layers * SP_COUNT && !P.failed; ++i) {
+            for (int i = 0; i < a.n_layers * SP_COUNT; ++i) {
                 const int l = i / SP_COUNT, ph = i % SP_COUNT;
-                if (ph == SP_O) S::produce_kv(args, P, l, rg);
-                if (rg.nb[ph] && !P.failed) S::produce_gemv(args, P, ph, l, rg.nb[ph]);
+                if (ph == SP_O && !S::produce_kv(args, P, l, rg)) break;
+                if (rg.nb[ph] && !S::produce_gemv(args, P, ph, l, rg.nb[ph], scales)) break;
             }
-            P.report(a.err);
+            S::land(a, P, scales);
+            step_report(a.err);
         }
         return;
     }
@@ -834,13 +862,12 @@ __global__ void __launch_bounds__(kStepThreads, 1) step_layers_kernel(const __gr
         // q/k/v phase begins, the residual in a CTA whose first work is the output projection.
         consumer_sync(kStepConsumers);
     }
-    StepRing R{0u, 0u, 0u, 0u, 0u};
-    const uint32_t seq0 = *a.epoch * kSeqPerStep;
+    StepRing R{0u, 0u, 0u};
     // One copy of the code for the four matrix phases: it has to fit the instruction cache.
 #pragma unroll 1
     for (int i = 0; i < a.n_layers * SP_COUNT; ++i) {
         const int l = i / SP_COUNT, ph = i % SP_COUNT;
-        const uint32_t seq = seq0 + (uint32_t)l + 1u;
+        const uint32_t seq = S::core().seq0 + (uint32_t)l + 1u;
         if (ph == SP_QKV && warp == kStepWarps - 1 && (int)blockIdx.x == l % (int)gridDim.x && l + 1 < a.n_layers) {      // the small tensors of the layer ahead come to L2 before their first use
 #pragma unroll 1
             for (int k = 0; k < 5; ++k) {
@@ -853,13 +880,13 @@ __global__ void __launch_bounds__(kStepThreads, 1) step_layers_kernel(const __gr
         const typename S::Range& rg = S::range(a);
         if (ph == SP_O) {
             if (rg.any) S::attend(seq, l == a.n_layers - 1, R);
-            if (rg.fold_head >= 0) S::fold(l, seq, rg.fold_head, R);
+            if (rg.fold_head >= 0) S::fold(l, seq, rg.fold_head);
             // Both end with a few warps reading the area that the output projection's input is staged in, whose first words may be other heads'.
             if (rg.any || rg.fold_head >= 0) consumer_sync(kStepConsumers);
         }
         if (rg.nb[ph]) S::gemv(ph, rg.nb[ph], l, seq, R);
     }
-    R.report(a.err);
+    step_report(a.err);
 }
 
 template <int Q>

@@ -6,6 +6,8 @@
 
 namespace cq {
 
+constexpr unsigned kStepWaitCycles = 2000000000u;      // about a second, and less than the 32-bit counter's period
+
 enum StepMat : int { SM_Q = 0, SM_K, SM_V, SM_O, SM_GATE, SM_UP, SM_DOWN, SM_COUNT };
 enum StepPhase : int { SP_QKV = 0, SP_O, SP_MLP, SP_DOWN, SP_COUNT };
 
@@ -31,6 +33,7 @@ struct StepCore {                    // everything but the tensor maps; the kern
     StepGemv g[SP_COUNT];
     int n_layers, dim, inter, n_heads, n_kv, grp, hd, max_seq, nsplit, staged_h;
     float eps, inv_dim, scale_log2, theta;
+    unsigned wait_cycles, started, expired, seq0;   // bound of the waits, in SM cycles; in a CTA's copy: when it began, the code of the first wait that expired, the step's first sequence number less one
     int off_x, off_corr, off_red, off_rms, off_cur, off_job, off_zero, off_q, off_hbuf, off_res, off_rope, off_range, off_ring, slots, slot_bytes, off_bars, smem;
 };
 struct alignas(64) StepArgs {

@@ -168,6 +168,10 @@ int cuqwen_get_params(const cuqwen_engine* e, cuqwen_params* out);
 uint64_t cuqwen_step_bytes(const cuqwen_engine* e, int ctx);
 /* Kernel launches in one decode step. */
 int cuqwen_step_launches(const cuqwen_engine* e);
+/* Test hook: how long after its start the kernel that runs all layers of a step ends its waits, in SM cycles (0 = the default and the most, 2e9: about a
+ * second).  A step whose waits expire ends with CUQWEN_ERR_TIMEOUT and leaves a wrong row in the cache; the engine goes on.  CUQWEN_ERR_STATE where
+ * an engine's layers are separate kernels. */
+int cuqwen_set_wait_cycles(cuqwen_engine* e, unsigned cycles);
 /* Tracing aid (no counterpart in the reference, whose benchmark/kernel_profile.cu times kernels in isolation): run ONE
  * step launch by launch with a CUDA event after every launch and return the microseconds between consecutive events,
  * in launch order (embedding, then per layer qkv / attention / o_proj / gate-up / down, lm_head, penalty, sampler;

@@ -1,6 +1,7 @@
 """A step whose layers are one kernel, against the oracle and against the launch-by-launch step of the same model, at the sizes where its work split, its ring
 and its key ranges have their edges."""
 import ctypes
+import time
 
 import numpy as np
 import pytest
@@ -156,3 +157,34 @@ def test_steps_at_changing_places(built, tmp_path, quant, dim, inter, heads, kv,
             assert np.array_equal(g.view(np.uint16), w.view(np.uint16)), places[i]
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("quant,hd", [(2, 64), (1, 128), (0, 128)])
+@pytest.mark.parametrize("cycles", [1, 20000])
+def test_waits_that_expire(built, tmp_path, quant, hd, cycles):
+    """Waits that end before the words and copies that they are for are there (at their first look; in the middle of the step, which takes some 100,000 cycles): the step, also one that feeds itself,
+    ends with an error and in time, and the next one, with waits of the usual length, is the same as an undisturbed engine's."""
+    cfg = dict(vocab=512, dim=512, inter=1024, layers=6, heads=4, kv=2, hd=hd, tied=True)
+    path = tmp_path / "m.bin"
+    binfmt.write_model(path, cfg, quant, binfmt.random_tensors(cfg, 5))
+    e, whole = make(cfg, quant, path), make(cfg, quant, path)
+    for ctx in (40, 1200):
+        whole.kv_fill_normal(ctx, 7)
+        whole.step(5, ctx)
+        _abi.check(_abi.lib().cuqwen_set_wait_cycles(e._h, cycles))
+        for _ in range(3):
+            e.kv_fill_normal(ctx, 7)
+            begin = time.perf_counter()
+            for call in (lambda: e.step(5, ctx), lambda: e.decode_n(5, ctx, 4)):
+                with pytest.raises(_abi.CuQwenError) as err:
+                    call()
+                assert err.value.code == 9
+            assert time.perf_counter() - begin < 5
+        _abi.check(_abi.lib().cuqwen_set_wait_cycles(e._h, 0))
+        e.kv_fill_normal(ctx, 7)
+        e.step(5, ctx)
+        for which in ("LOGITS", "KEY_CACHE"):
+            got, want = (x.read(which).reshape(-1) if which == "LOGITS" else x.read(which).reshape(6, 2, MAX_SEQ, hd)[:, :, :ctx + 1] for x in (e, whole))
+            assert np.array_equal(got.view(np.uint16), want.view(np.uint16)), which
+    e.close()
+    whole.close()

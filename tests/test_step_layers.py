@@ -47,3 +47,24 @@ def test_no_variant_spills():
         pytest.skip("the library was not built here")
     spills = re.findall(r"(\d+) bytes spill stores, (\d+) bytes spill loads", "".join(p.read_text() for p in logs))
     assert spills == [("0", "0")] * 6
+
+
+def test_the_bound_of_its_waits(run, tmp_path):      # noqa: F811
+    """Set for the kernel alone; the graph that holds it is captured anew."""
+    path = tmp_path / "m.bin"
+    binfmt.write_model(path, PLAIN, 2, binfmt.random_tensors(PLAIN, 3))
+    run("""
+stub.stub_sms(148)
+from cuqwen_b200 import _abi
+def make(flags):
+    p = E.custom_params(512, 256, 512, 2, 4, 2, 64, 2, max_seq_len=256)
+    p.flags = flags
+    eng = E.Engine(p)
+    eng.load(sys.argv[1])
+    return eng
+one, many = make(E.FLAG_NO_GRAPH), make(E.FLAG_NO_GRAPH | E.FLAG_NO_HANDOVER)
+code = lambda e, n: _abi.lib().cuqwen_set_wait_cycles(e._h, n)
+assert [code(one, n) for n in (0, 1, 2000000000, 2000000001)] == [0, 0, 0, 1] and code(many, 5) == 8
+one.step(1, 0)
+assert one.step_launches == 5
+""", path)
