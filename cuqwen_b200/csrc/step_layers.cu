@@ -15,7 +15,7 @@ int launch_step_layers(int quant, const StepArgs& a, const LaunchCfg& cfg) {
     return quant == Q_I4 ? launch_step_layers_i4(a, cfg) : quant == Q_I8 ? launch_step_layers_i8(a, cfg) : launch_step_layers_f16(a, cfg);
 }
 
-static constexpr int kWarps = 16, kBars = 32, kSmem = 227 * 1024;
+static constexpr int kWarps = kStepWarps, kSmem = 227 * 1024;
 
 static int unit_bytes(int quant) { return quant == Q_I4 ? 64 : 128; }       // of one row: 128 columns quantised, 64 columns fp16
 static int unit_cols(int quant) { return quant == Q_F16 ? 64 : 128; }
@@ -59,9 +59,9 @@ bool step_layers_plan(const StepShape& s, StepCore& a, size_t (&words)[7]) {
         for (g.ks = 0; 1 << g.ks < g.kp;) ++g.ks;
         const int U = K / unit_cols(s.quant);
         int u = a.slot_bytes / (mt * rows * gb);
+        if (u * gb / 64 > 256) u = 256 * 64 / gb;                        // (a copy's box; before the next line, as stages of several K-parts hold whole rounds of them)
         if (u > g.kp) u = u / g.kp * g.kp;
         if (u > U) u = U;
-        if (u * gb / 64 > 256) u = 256 * 64 / gb;
         g.U = U; g.ustride = gb * rows; g.units = u; g.nst = (U + u - 1) / u;
         g.box_bytes = rows * u * gb; g.stage_bytes = mt * g.box_bytes;
         g.scale_bytes = q ? mt * rows * (K / kGroup) * 2 : 0;
@@ -73,21 +73,21 @@ bool step_layers_plan(const StepShape& s, StepCore& a, size_t (&words)[7]) {
     // shared memory: the staged vector (digits or fp16) with the attention's merge buffers over it, small areas, scales, ring, barriers
     int K = s.dim > qd ? s.dim : qd;
     if (s.inter > K) K = s.inter;
-    const int merge = 8 * (s.hd / 16 * 512 + 256), states = 8 * kMaxGroup * (s.hd + 2) * 4, folds = kWarps * (s.hd + 2) * 4;
+    const int merge = 8 * (s.hd / 16 * 512 + 256), folds = kWarps * (s.hd + 2) * 4;
     int area = 2 * K, o = (int)sizeof(StepCore);
-    for (int m : {merge, states, folds}) if (area < m) area = m;
+    for (int m : {merge, folds}) if (area < m) area = m;
     auto take = [&](int bytes, int align) { o = (o + align - 1) / align * align; const int at = o; o += bytes; return at; };
     a.off_x = take(area, 128);
-    a.off_corr = take(K / kGroup * 8, 16); a.off_job = take(SP_COUNT * kWarps * 16, 16);
-    a.off_zero = take(256, 16); a.off_red = take(2 * kWarps * 17 * 4, 16); a.off_rms = take(kWarps * 4, 16);
+    a.off_corr = take(K / kGroup * 8, 16); a.off_job = take(SP_COUNT * kWarps * kStepJobBytes, 16);
+    a.off_zero = take(256, 16); a.off_red = take(2 * kWarps * kStepRed * 4, 16); a.off_rms = take(kWarps * 4, 16);
     a.off_q = take(kMaxGroup * (s.hd * 2 + 64), 16); a.off_cur = take(s.hd == 128 ? 32 * 128 + 256 : 256, 128); a.off_hbuf = take(256 + 264 + 8, 16);
-    a.off_res = take(a.g[SP_O].nb * rows_out * 2, 16); a.off_rope = take(a.g[SP_QKV].nb * 16 * 8, 16); a.off_range = take(64, 16);
+    a.off_res = take(a.g[SP_O].nb * rows_out * 2, 16); a.off_rope = take(a.g[SP_QKV].nb * 16 * 8, 16); a.off_range = take(kStepRangeBytes, 16);
     for (int i = 0; i < SP_COUNT; ++i) a.g[i].off_scale = take(a.g[i].nb * a.g[i].scale_bytes, 128);
     a.off_ring = take(0, 1024);            // (the swizzle's pattern)
-    const int bars = (2 * kBars + 2 * SP_COUNT) * 8;
+    const int bars = (2 * kStepBars + 2 * SP_COUNT) * 8;
     // a tile's last rows may lie beyond its block: their loads run up to 15 rows past the last stage, their scales up to 15 rows past the scales (into the ring)
     a.slots = (kSmem - o - 1024 - bars) / a.slot_bytes;
-    if (a.slots > 16) a.slots = 16;
+    if (a.slots > kStepBars / 2) a.slots = kStepBars / 2;
     if (a.slots < 4) return false;
     a.off_bars = a.off_ring + a.slots * a.slot_bytes + 1024; a.smem = a.off_bars + bars;
     for (const StepGemv& g : a.g) if (g.stage_bytes > a.slot_bytes || g.units < 1 || g.brows << g.ks > 32 * kWarps) return false;

@@ -31,9 +31,7 @@
 
 namespace cq {
 
-constexpr int kStepWarps = 16, kStepConsumers = kStepWarps * 32, kStepThreads = kStepConsumers + 128;      // the producer has a warpgroup to itself, whose registers the consumers take over
-constexpr int kStepRed = 17;                  // floats of a warp's sixteen sums, with one between so that K-parts lie in different banks
-constexpr int kStepBars = 32;                 // pairs of stage barriers: twice the slots of the ring, at least
+constexpr int kStepConsumers = kStepWarps * 32, kStepThreads = kStepConsumers + 128;      // the producer has a warpgroup to itself, whose registers the consumers take over
 
 template <int Q> struct StepUnit;             // bytes of a row's column unit
 template <> struct StepUnit<Q_I4> { static constexpr int GB = 64, COLS = 128; };
@@ -118,9 +116,11 @@ struct StepLayers {
     static __device__ __forceinline__ uint32_t bar_sempty(const StepCore& a, int ph) { return smem_u32(step_smem) + a.off_bars + (2 * kStepBars + SP_COUNT + ph) * 8; }
     // What every layer needs to know, computed once: the attention's key range, the head to merge, the blocks of each phase.
     struct Range { int kvh, split, t0, t1c, nstage, any, own, nne; int pos, fold_head; int nb[SP_COUNT]; };
+    static_assert(sizeof(Range) <= kStepRangeBytes, "");
     static __device__ __forceinline__ const Range& range(const StepCore& a) { return *reinterpret_cast<const Range*>(step_smem + a.off_range); }
     // A warp's part of a phase's blocks: byte offset of its tile in a stage, of its tile's first scale row in a block's scales, its K-part (or none).
-    struct Job { int in_stage, scales, part, tile; };
+    struct alignas(kStepJobBytes) Job { int in_stage, scales, part; };
+    static_assert(sizeof(Job) == kStepJobBytes, "");
     static __device__ __forceinline__ Job& job(const StepCore& a, int ph, int warp) { return reinterpret_cast<Job*>(step_smem + a.off_job)[ph * kStepWarps + warp]; }
 
     template <class T> static __device__ __forceinline__ const T* at_layer(const StepCore& a, const T* p, int l) { return reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + (size_t)l * a.layer_stride); }
@@ -820,7 +820,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) step_layers_kernel(const __gr
         const int ph = tid / kStepWarps, w = tid % kStepWarps;
         const StepGemv& G = a.g[ph];
         const int tile = w % G.nt, part = w / G.nt, m = tile / G.rt, r = tile - m * G.rt;
-        S::job(a, ph, w) = typename S::Job{m * G.box_bytes + r * 16 * kChunkBytes, (m * G.brows + r * 16) * G.ngrp * 2, part < G.kp ? part : 1 << 30, tile};
+        S::job(a, ph, w) = typename S::Job{m * G.box_bytes + r * 16 * kChunkBytes, (m * G.brows + r * 16) * G.ngrp * 2, part < G.kp ? part : 1 << 30};
     }
     __syncthreads();
     // 640 threads are launched with 96 registers each, 61,440; 512 x 112 + 128 x 32 are as many

@@ -6,6 +6,11 @@
 
 namespace cq {
 
+// What the kernel and the host's map of its shared memory have in common.
+constexpr int kStepWarps = 16;                // consumer warps
+constexpr int kStepRed = 17;                  // floats of a warp's sixteen sums, with one between so that K-parts lie in different banks
+constexpr int kStepBars = 32;                 // pairs of stage barriers: twice the slots of the ring, at least
+constexpr int kStepRangeBytes = 64, kStepJobBytes = 16;
 constexpr unsigned kStepWaitCycles = 2000000000u;      // about a second, and less than the 32-bit counter's period
 
 enum StepMat : int { SM_Q = 0, SM_K, SM_V, SM_O, SM_GATE, SM_UP, SM_DOWN, SM_COUNT };

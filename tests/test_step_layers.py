@@ -1,5 +1,7 @@
 """Which engines run a step's layers as one kernel, and which launch by launch, on the CPU over tests/cudart_stub.cpp."""
 import re
+import subprocess
+from pathlib import Path
 
 import pytest
 
@@ -68,3 +70,14 @@ assert [code(one, n) for n in (0, 1, 2000000000, 2000000001)] == [0, 0, 0, 1] an
 one.step(1, 0)
 assert one.step_launches == 5
 """, path)
+
+
+def test_every_plan_is_one_that_the_kernel_can_run(built, tmp_path):
+    """Alignment and sizes of copies, stages inside their slots, areas of shared memory, over the widths, head counts and SM counts that the plan takes."""
+    exe = tmp_path / "probe"
+    lib = build.LIB.parent
+    r = subprocess.run(["g++", "-std=c++17", "-O1", f"-I{build.cuda_home() / 'include'}", str(Path(__file__).parent / "step_plan_probe.cpp"), "-o", str(exe), f"-L{lib}", "-lcuqwen_b200", f"-Wl,-rpath,{lib}",
+                        f"-L{build.cuda_home() / 'lib64'}", "-lcudart"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
