@@ -2,6 +2,7 @@
 and its key ranges have their edges."""
 import ctypes
 import time
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
@@ -89,6 +90,31 @@ def test_against_the_oracle(built, tmp_path, name, quant):
     orc.close()
 
 
+@pytest.mark.parametrize("name", ["0.5b", "wide attention"])
+@pytest.mark.parametrize("quant", [0, 1, 2])
+def test_long_contexts_against_the_oracle(built, tmp_path, name, quant):
+    """The last context of one key range a KV head, and several ranges (18 or 74 at most), whose partials travel between CTAs and are merged: the oracle goes on from the engine's own filled cache."""
+    cfg = MODELS[name]
+    path = tmp_path / "m.bin"
+    binfmt.write_model(path, cfg, quant, binfmt.random_tensors(cfg, 6))
+    eng, orc = make(cfg, quant, path), O.OracleModel(str(path), MAX_SEQ)
+    shape = (cfg["layers"], cfg["kv"], MAX_SEQ, cfg["hd"])
+    eng.kv_fill_normal(MAX_SEQ, 7)
+    for view, which in zip(orc.kv_views(), ("KEY_CACHE", "VALUE_CACHE")):
+        view[...] = eng.read(which).reshape(shape)
+    for ctx in (255, 256, 700, 1599):
+        eng.step(3 + ctx % 100, ctx)
+        orc.step(3 + ctx % 100, ctx)
+        assert close(eng.read("LOGITS"), orc.logits), (ctx, report(eng.read("LOGITS"), orc.logits))
+        for view, which in zip(orc.kv_views(), ("KEY_CACHE", "VALUE_CACHE")):
+            got = eng.read(which).reshape(shape)[:, :, ctx]
+            assert close(got, view[:, :, ctx]), (ctx, which, report(got, view[:, :, ctx]))
+            view[:, :, ctx] = got                      # each step over the same cache
+    assert eng.step_launches == 5
+    eng.close()
+    orc.close()
+
+
 def test_steps_of_two_engines_do_not_mix(built, tmp_path):
     """Their exchange words are their own, and a step's numbers go on when the control block is written anew (decode_n, a profile, which runs the separate launches)."""
     cfg = MODELS["0.5b"]
@@ -107,6 +133,26 @@ def test_steps_of_two_engines_do_not_mix(built, tmp_path):
     got += b.decode_n(got[-1], 16, 8).tolist()
     assert got == want
     for e in (a, b, c):
+        e.close()
+
+
+def test_engines_in_two_threads(built, tmp_path):
+    """A step's kernel takes the whole GPU, all of it at once: engines that are called from several threads go one step at a time, and each gets what it gets alone."""
+    cfg = MODELS["0.5b"]
+    path = tmp_path / "m.bin"
+    binfmt.write_model(path, cfg, 2, binfmt.random_tensors(cfg, 9))
+
+    def tokens(e, first):
+        out = [e.step(first, 0)]
+        for i in range(1, 60):
+            out.append(e.step(out[-1], i))
+        return out + e.decode_n(out[-1], 60, 100).tolist() + e.step_loop(7, 160, 60).tolist()
+
+    engines = [make(cfg, 2, path) for _ in range(3)]
+    alone = [tokens(e, 5 + i) for i, e in enumerate(engines)]
+    with ThreadPoolExecutor(len(engines)) as ex:
+        assert list(ex.map(tokens, engines, range(5, 8))) == alone
+    for e in engines:
         e.close()
 
 
