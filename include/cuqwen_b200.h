@@ -39,13 +39,16 @@ enum { CUQWEN_FP16 = 0, CUQWEN_INT8 = 1, CUQWEN_INT4 = 2 };          /* include/
 enum { CUQWEN_MODEL_0_5B = 0, CUQWEN_MODEL_1_5B = 1, CUQWEN_MODEL_3B = 2, CUQWEN_MODEL_7B = 3, CUQWEN_MODEL_14B = 4, CUQWEN_MODEL_CUSTOM = -1 };
 
 enum {
-    CUQWEN_FLAG_ACCURATE_ROPE = 1,  /* accurate pow/sin/cos instead of the fast-math forms the reference build uses */
+    CUQWEN_FLAG_ACCURATE_ROPE = 1,  /* accurate pow/sin/cos instead of the fast-math forms the reference build uses; for comparisons kernel by kernel: a step of such
+                                     * an engine is a launch for every kernel and takes 1.1 to 1.6 times as long as one whose layers are one kernel */
     CUQWEN_FLAG_NO_PDL = 2,         /* plain stream order between kernels (no programmatic dependent launch) */
     CUQWEN_FLAG_NO_GRAPH = 4,       /* launch the step kernel by kernel instead of replaying a CUDA graph */
-    /* 8 is unused (it selected a persistent one-launch step kernel that was removed: it never beat the launch chain) */
-    CUQWEN_FLAG_STEP_TRACE = 16,    /* profiling: every GEMV / attention launch of a step stamps its timeline (CUQWEN_PTR_STEP_TRACE) */
+    CUQWEN_FLAG_SEPARATE_KERNELS = 8, /* a launch for every kernel of a step instead of one kernel for all its layers.  That one takes all SMs at once: engines that share
+                                     * a GPU go one step at a time, and each is faster alone, but together they get through 5 to 8 % less than with this flag */
+    CUQWEN_FLAG_STEP_TRACE = 16,    /* profiling: the step is launched kernel by kernel, every GEMV / attention launch stamps its timeline (CUQWEN_PTR_STEP_TRACE) */
     CUQWEN_FLAG_TP_NCCL = 32,       /* tensor parallel: sum the row-parallel partials with NCCL all-reduce calls instead of peer stores */
-    CUQWEN_FLAG_NO_HANDOVER = 64,   /* o_proj and the down projection convert their input themselves instead of taking it staged from the attention fold / the SwiGLU kernel */
+    CUQWEN_FLAG_NO_HANDOVER = 64,   /* o_proj and the down projection convert their input themselves instead of taking it staged from the attention fold / the SwiGLU kernel;
+                                     * the step is then launched kernel by kernel */
     CUQWEN_FLAG_PREFILL_ATTN_MMA = 512, /* cuqwen_prefill: attention on the mma.sync kernel at every length (comparison variant); without it that kernel takes
                                      * the portions that fill few SMs, with head_dim 128 up to 512 keys, and the tcgen05 kernel the others */
     CUQWEN_FLAG_TP_SUM_IN_GEMV = 256, /* tensor parallel, peer-store exchange: no separate sum kernel; every CTA of the GEMV that consumes the
@@ -150,7 +153,7 @@ enum {
                                      * wait returned, last input staged, last main loop done, last exit, 2 spare ("~" = stored complemented).
                                      * Stamps accumulate: zero the block between steps. */
     CUQWEN_PTR_TOKEN, CUQWEN_PTR_POS, CUQWEN_PTR_HISTORY_LEN, CUQWEN_PTR_SAMPLED,   /* the four device ints a step reads / writes (QwenState::d_token, d_pos, d_history_len, d_sampled_token) */
-    CUQWEN_PTR_PARTIAL_O, CUQWEN_PTR_PARTIAL_ML,   /* split-KV scratch: fp32 partial outputs, (max, sum) pairs */
+    CUQWEN_PTR_PARTIAL_O, CUQWEN_PTR_PARTIAL_ML,   /* split-KV scratch of a step launched kernel by kernel: fp32 partial outputs, (max, sum) pairs */
     CUQWEN_PTR_UP, CUQWEN_PTR_MLP_OUT,              /* QwenState::up / mlp_out: allocated for harnesses that write them, unused by the step (as in the reference, src/model.cu:18-20) */
     CUQWEN_PTR_STREAM,                              /* not a buffer: the cudaStream_t the engine queues its steps on (bytes = 0) */
     CUQWEN_PTR_KEY_SCALE, CUQWEN_PTR_VALUE_SCALE,   /* CUQWEN_FLAG_KV_INT8: fp32 [n_layers][n_kv_heads][max_seq_len] row scales; the caches are then int8 in the same layout */
@@ -166,14 +169,16 @@ int cuqwen_get_params(const cuqwen_engine* e, cuqwen_params* out);
 /* Algorithmic bytes one decode step reads at context length ctx on this rank: all weights, scales, biases,
  * norms, one embedding row, and K+V rows [0, ctx) of every layer. */
 uint64_t cuqwen_step_bytes(const cuqwen_engine* e, int ctx);
-/* Kernel launches in one decode step. */
+/* Kernel launches in one decode step: 5 where its layers are one kernel (one GPU, fp16 cache, none of the flags ACCURATE_ROPE, SEPARATE_KERNELS, STEP_TRACE and NO_HANDOVER, and at most one attention
+ * CTA for each SM), else 1 + 6 n_layers + 3 and, with tensor parallelism, the exchanges'. */
 int cuqwen_step_launches(const cuqwen_engine* e);
 /* Test hook: how long after its start the kernel that runs all layers of a step ends its waits, in SM cycles (0 = the default and the most, 2e9: about a
  * second).  A step whose waits expire ends with CUQWEN_ERR_TIMEOUT and leaves a wrong row in the cache; the engine goes on.  CUQWEN_ERR_STATE where
  * an engine's layers are separate kernels. */
 int cuqwen_set_wait_cycles(cuqwen_engine* e, unsigned cycles);
 /* Tracing aid (no counterpart in the reference, whose benchmark/kernel_profile.cu times kernels in isolation): run ONE
- * step launch by launch with a CUDA event after every launch and return the microseconds between consecutive events,
+ * step kernel by kernel with a CUDA event after every launch and return the microseconds between consecutive events - also on
+ * an engine whose cuqwen_step runs all layers as one kernel (cuqwen_step_launches: 5), which these times do not describe -
  * in launch order (embedding, then per layer qkv / attention / o_proj / gate-up / down, lm_head, penalty, sampler;
  * tensor-parallel runs add their exchange launches).  Times include launch gaps.  Every rank must call it together. */
 int cuqwen_step_profile(cuqwen_engine* e, int token, int pos, float* us, int cap, int* n_out);

@@ -136,8 +136,9 @@ def test_steps_of_two_engines_do_not_mix(built, tmp_path):
         e.close()
 
 
-def test_engines_in_two_threads(built, tmp_path):
-    """A step's kernel takes the whole GPU, all of it at once: engines that are called from several threads go one step at a time, and each gets what it gets alone."""
+@pytest.mark.parametrize("flags", [0, E.FLAG_SEPARATE_KERNELS])
+def test_engines_in_several_threads(built, tmp_path, flags):
+    """A step's kernel takes the whole GPU, all of it at once: engines that are called from several threads go one step at a time, or share it kernel by kernel, and each gets what it gets alone."""
     cfg = MODELS["0.5b"]
     path = tmp_path / "m.bin"
     binfmt.write_model(path, cfg, 2, binfmt.random_tensors(cfg, 9))
@@ -148,8 +149,9 @@ def test_engines_in_two_threads(built, tmp_path):
             out.append(e.step(out[-1], i))
         return out + e.decode_n(out[-1], 60, 100).tolist() + e.step_loop(7, 160, 60).tolist()
 
-    engines = [make(cfg, 2, path) for _ in range(3)]
+    engines = [make(cfg, 2, path, flags) for _ in range(3)]
     alone = [tokens(e, 5 + i) for i, e in enumerate(engines)]
+    assert {e.step_launches for e in engines} == {1 + 6 * cfg["layers"] + 3 if flags else 5}
     with ThreadPoolExecutor(len(engines)) as ex:
         assert list(ex.map(tokens, engines, range(5, 8))) == alone
     for e in engines:

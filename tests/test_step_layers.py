@@ -36,7 +36,7 @@ def test_the_layers_of_a_step_are_one_launch(run, tmp_path, quant, hd):     # no
     assert len(names) == 5 and "step_layers_kernel" in names[1] and " 148,1,1 " in names[1] and "gemv_kernel" in names[2]
 
 
-@pytest.mark.parametrize("flags,splits,sms", [("E.FLAG_ACCURATE_ROPE", 0, 148), ("E.FLAG_NO_HANDOVER", 0, 148), ("E.FLAG_STEP_TRACE", 0, 148), ("E.FLAG_KV_INT8", 0, 148),
+@pytest.mark.parametrize("flags,splits,sms", [("E.FLAG_ACCURATE_ROPE", 0, 148), ("E.FLAG_SEPARATE_KERNELS", 0, 148), ("E.FLAG_NO_HANDOVER", 0, 148), ("E.FLAG_STEP_TRACE", 0, 148), ("E.FLAG_KV_INT8", 0, 148),
                                               ("0", 75, 148), ("0", 0, 3)])
 def test_what_the_kernel_does_not_know_stays_launch_by_launch(run, tmp_path, flags, splits, sms):      # noqa: F811
     assert "step_layers_kernel" not in kernels_of_a_step(run, tmp_path, PLAIN, 2, flags, splits, sms)
