@@ -6,8 +6,10 @@
 One "step" is one decode token (one pass of the hot path).  Rank 0 prints ONE JSON line:
   value   tokens/s with the token fed back on the device (cuqwen_decode_n: K graph replays between two CUDA events)
   e2e     tokens/s through cuqwen_step, the call a host makes per token: host token in (H2D), sampled token out (D2H)
-  roofline    the dominant kernel (gate/up W4A16 GEMV + SwiGLU) timed alone over all layers' weights, algorithmic
-              bytes / CUDA-event time against the measured HBM copy bandwidth; `step` gives the same for the whole step
+  roofline    the timed step, whose layers are one kernel: algorithmic bytes / CUDA-event time against the measured HBM
+              copy bandwidth (also under `step`).  Where a step is separate launches (several GPUs, 8-bit cache): its
+              dominant kernel, the gate/up W4A16 GEMV + SwiGLU, timed alone over all layers' weights; `gate_up_kernel`
+              has that in any case
   cpu_baseline  the scalar CPU oracle of the same step on the host cores (N=1, rank 0, bounded sample)
 --impl reference times the reference's own CUDA build (oracle/_ref, its qwen_forward loop) on the same file and context.
 Under torchrun (N>1) the model is tensor-parallel over the N GPUs (strong scaling: the work per token is fixed).
@@ -342,9 +344,15 @@ def run_ours(a):
     if rank == 0:
         alg, sec = dominant_kernel_roofline(eng, E, K, cfg, qid)
         ach = alg / sec / 1e9
-        out["roofline"] = {"bound": "hbm", "kernel": "gemv_kernel<int4, SWIGLU> (gate/up GEMV + SwiGLU)", "achieved": round(ach, 1), "peak": peak,
-                           "unit": "GB/s", "frac": round(ach / peak, 4), "peak_source": peak_src + ", of measured", "frac_of_nominal_8tbs": round(ach / 8000.0, 4), "bytes_per_launch": alg,
-                           "us_per_launch": round(sec * 1e6, 3), "traffic": NCU_TRAFFIC_BYTES.get((a.model, a.quant))}
+        one_kernel = eng.step_launches == 5
+        gate_up = {"bound": "hbm", "kernel": "gemv_kernel<int4, SWIGLU> (gate/up GEMV + SwiGLU)", "in_timed_step": not one_kernel, "achieved": round(ach, 1), "peak": peak,
+                   "unit": "GB/s", "frac": round(ach / peak, 4), "peak_source": peak_src + ", of measured", "frac_of_nominal_8tbs": round(ach / 8000.0, 4), "bytes_per_launch": alg,
+                   "us_per_launch": round(sec * 1e6, 3), "traffic": NCU_TRAFFIC_BYTES.get((a.model, a.quant))}
+        out["gate_up_kernel"] = gate_up
+        out["roofline"] = gate_up if not one_kernel else {
+            "bound": "hbm", "kernel": f"step_layers_kernel<{a.quant}, {cfg['hd']}> (all layers) and the step's four other launches (embedding, lm_head, penalty, argmax)", "in_timed_step": True,
+            "achieved": round(step_gbs, 1), "peak": peak, "unit": "GB/s", "frac": round(step_gbs / peak, 4), "peak_source": peak_src + ", of measured", "frac_of_nominal_8tbs": round(step_gbs / 8000.0, 4),
+            "bytes_per_launch": step_bytes_total, "us_per_launch": round(ms / Kst * 1e3, 3), "traffic": None}
     par = None if (a.no_parity or a.layers) else parity_leg(eng, a, cfg, path, rank, world, local, dist)
     if rank == 0 and par is not None:
         out["parity"] = par

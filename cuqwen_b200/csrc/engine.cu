@@ -383,8 +383,8 @@ static int walk_file(cuqwen_engine* e, Cursor cur, Arena& ar, int lm_fmt) {
 // Prepares the step whose layers are one kernel (step_layers.h), where this engine can take it; the launch-by-launch step stays with a flag that asks for it; with tensor parallelism and the
 // 8-bit cache, whose exchanges and rows the kernel does not know; with a timeline or a switched-off hand-over, which speak of the separate launches; with the accurate rotation, the mode
 // in which kernels are compared with the oracle one by one; with shapes beyond the plan; on a device without cooperative launches.
-// No size of the table's models is slower than by separate launches (0.5B to 14B, each format, 1 to 31,900 keys): int4 and int8 1.06 to 1.65 times as fast, fp16 1.05 to 1.40 up to 3B and
-// 1.00 to 1.03 at 7B and 14B, whose matrices stream for long enough that little is left between them.
+// No size of the table's models is slower than by separate launches (0.5B to 14B, each format, 100 to 31,900 keys): int4 and int8 1.09 to 1.64 times as fast, fp16 1.06 to 1.40 up to 3B,
+// 1.00 to 1.01 at 7B and 1.02 at 14B, whose matrices stream for long enough that little is left between them.
 static int prepare_layers(cuqwen_engine* e) {
     const cuqwen_params& p = e->p;
     int coop = 0;

@@ -13,16 +13,17 @@
 // residual, gate/up + SwiGLU, down projection + residual.  A CTA keeps the residual of its own rows in shared memory (the two row-parallel projections are cut
 // alike).  CTAs without work in a phase do not read its input.
 //
-// Measured, us a step, launch by launch -> here (one B200, the same box): 0.5B int4 at 255 keys 677 -> 434, 0.5B fp16 at 1777 655 -> 498, 7B int4 at 8192 1462 -> 1104, six 14B int8 layers
-// at 31,999 691 -> 603.  What the phases take, in cycles of 1.9 GHz (0.5B int4 / 7B int4): hand-over, from one phase's end until its words are here, 2000 / 2000 to 2500; a vector to digits
-// 370 / 740 and its norm 250; products 1150 / 2780 (q/k/v), 16,800 (7B gate/up, 70 MB), 11,600 (down); a block's finish 800 to 1300; attention 6400 / 7300, of which the tile loop
-// 2800 / 3800; merge of the partials, 7B, 5500 to 8500.  The 7B layer's bytes alone would take 39,000 of its 69,000 cycles.
+// Measured, us a step, launch by launch -> here (one B200, in turn on the same box): 0.5B int4 at 255 keys 679 -> 428, 0.5B fp16 at 1777 with the penalty 660 -> 488, 7B int4 at 8192 1489 -> 1102, six 14B
+// int8 layers at 31,999 688 -> 625.  What the phases take, in cycles of 1.9 GHz (0.5B int4 at 255 keys / 7B int4 at 8192, one thread's stamps, median of the CTAs): words from one phase's end until they
+// are here 1600 to 1700 / 1800 to 2300; a vector to digits, or SwiGLU's digits to shared memory, 650 to 2400 / 1000 to 1900; products of q/k/v 1140 / 2700, of o 950 / 2660, of gate/up 2260 / 16,500
+// (7B: 70 MB), of down 1820 / 10,950; a block's finish 930 to 1180 / 920 to 1460; attention: q 3500 / 2000, tiles 2700 / 3640, merge of the warps 2260 / 1990; merge of a head's partials 8700 (0.5B
+// at 1777 keys) / 5800.  A 7B layer takes 66,000 cycles, its bytes alone would take 39,000.
 // A warp's products of one group cost some 600 cycles next to the fifteen other warps' (operands from shared memory 390 and the integer MMAs 300), a chain, not a rate.  Slower were: the next
 // group's weights loaded ahead (7B 1094 -> 1240 us), two groups side by side (1173), rolled loops in the attention (1100 to 1135), a head's merge shared out among the CTAs that it has (1128),
 // polls through one lane a warp (1160) and weights asked into L2 ahead of the ring (1210).
 //
 // What this cost most to find: the consumers' code must fit the instruction caches (118 KB of phases inlined four times took 40 us a layer of the 0.5B model, 60 KB with one copy of
-// the phases 19), no register may spill (the spill lines' L1 is what 227 KB of shared memory leave, 28 KB; the 14B step 708 -> 637 us when most of them went), and keys and values
+// the phases 19), no register may spill (the spill lines' L1 is what 227 KB of shared memory leave, 28 KB; the 14B int8 step 708 -> 637 us, six fp16 layers of 3B 371 -> 340), and keys and values
 // must not collide in the banks (a tile 2300 -> 1500 cycles).
 #pragma once
 #include "attn_split.cuh"

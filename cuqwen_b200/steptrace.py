@@ -1,8 +1,11 @@
-"""Where one decode step spends its time.
+"""Where a decode step that is launched kernel by kernel spends its time.
 
-``python -m cuqwen_b200.steptrace --model 7b --quant int4 --ctx 8192`` prints two tables for a random-init model:
+An engine without flags runs all layers of a step as one kernel, which these instruments do not look into (its time is
+printed beside them); they describe the step of ``CUQWEN_FLAG_SEPARATE_KERNELS``, which is also that of tensor parallelism
+and of the 8-bit cache.  ``python -m cuqwen_b200.steptrace --model 7b --quant int4 --ctx 8192`` prints two tables for a
+random-init model:
 
-* launch by launch (``cuqwen_step_profile``): the default path run eagerly with a CUDA event after every launch, averaged
+* launch by launch (``cuqwen_step_profile``): the kernels run eagerly with a CUDA event after every launch, averaged
   per kind of kernel (times include launch gaps, so they bound the graph replay from above);
 * inside the graph (``CUQWEN_FLAG_STEP_TRACE``): every GEMV / attention launch stamps its own timeline while the step
   replays as a CUDA graph with programmatic dependent launch - relative to the moment the launch before it finished:
@@ -38,17 +41,23 @@ def model_file(model: str, quant: str, seed: int = 42) -> Path:
 
 def launches(model: str, quant: str, ctx: int, reps: int = 5) -> dict:
     cfg = binfmt.MODELS[model]
-    eng = E.Engine(E.model_params(model, quant))
-    eng.load(str(model_file(model, quant)))
-    eng.kv_fill_normal(ctx, 42)
-    eng.decode_n(1234, ctx, 64)
-    ms_graph = eng.last_decode_ms / 64
+    ms = []
+    for flags in (0, E.FLAG_SEPARATE_KERNELS):
+        prm = E.model_params(model, quant)
+        prm.flags = flags
+        eng = E.Engine(prm)
+        eng.load(str(model_file(model, quant)))
+        eng.kv_fill_normal(ctx, 42)
+        eng.decode_n(1234, ctx, 64)
+        ms.append(eng.last_decode_ms / 64)
+        if not flags:
+            eng.close()
     us = sum(eng.profile_step(5, ctx + 64 + i) for i in range(reps)) / reps
     L = cfg["layers"]
     per = (len(us) - 1 - 3) // L
     body = us[1:1 + per * L].reshape(L, per)
     names = ["qkv", "attention (2 launches)", "o_proj", "gate/up", "down"] if per == 5 else [f"k{i}" for i in range(per)]
-    out = {"graph_ms_per_step": ms_graph, "eager_sum_us": float(us.sum()), "embed": float(us[0]),
+    out = {"one_kernel_ms_per_step": ms[0], "graph_ms_per_step": ms[1], "eager_sum_us": float(us.sum()), "embed": float(us[0]),
            "per_layer": {n: float(v) for n, v in zip(names, body[1:].mean(0))},
            "tail": {n: float(v) for n, v in zip(["lm_head", "penalty", "argmax"], us[1 + per * L:])}}
     eng.close()
@@ -94,7 +103,7 @@ def main():
     a = ap.parse_args()
     la = launches(a.model, a.quant, a.ctx)
     print(f"Qwen2.5-{a.model} {a.quant}, KV context {a.ctx}")
-    print(f"default path: {la['graph_ms_per_step']:.3f} ms per step as a graph; launch by launch {la['eager_sum_us'] / 1e3:.3f} ms")
+    print(f"all layers as one kernel: {la['one_kernel_ms_per_step']:.3f} ms per step; separate kernels: {la['graph_ms_per_step']:.3f} ms as a graph, {la['eager_sum_us'] / 1e3:.3f} ms launch by launch")
     print(f"  embedding {la['embed']:.2f} us")
     for n, v in la["per_layer"].items():
         print(f"  {n:<22s} {v:7.2f} us per layer")

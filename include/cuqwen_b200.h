@@ -40,7 +40,7 @@ enum { CUQWEN_MODEL_0_5B = 0, CUQWEN_MODEL_1_5B = 1, CUQWEN_MODEL_3B = 2, CUQWEN
 
 enum {
     CUQWEN_FLAG_ACCURATE_ROPE = 1,  /* accurate pow/sin/cos instead of the fast-math forms the reference build uses; for comparisons kernel by kernel: a step of such
-                                     * an engine is a launch for every kernel and takes 1.1 to 1.6 times as long as one whose layers are one kernel */
+                                     * an engine is a launch for every kernel and takes up to 1.6 times as long as one whose layers are one kernel */
     CUQWEN_FLAG_NO_PDL = 2,         /* plain stream order between kernels (no programmatic dependent launch) */
     CUQWEN_FLAG_NO_GRAPH = 4,       /* launch the step kernel by kernel instead of replaying a CUDA graph */
     CUQWEN_FLAG_SEPARATE_KERNELS = 8, /* a launch for every kernel of a step instead of one kernel for all its layers.  That one takes all SMs at once: engines that share
